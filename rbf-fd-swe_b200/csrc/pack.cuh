@@ -8,8 +8,9 @@
 // device once and rearranged there by two kernels into every layout the stage
 // kernels read:
 //   * W / idx:   the 8-lanes-per-node layout (stage_kernel.cuh, stage_tma.cuh),
-//   * Wl / idxl: the tile-transposed node-per-lane layout (stage_lane.cuh), and
-//     idxs, the same indices as 16-bit offsets from each node's own row,
+//   * Wl / idxl: the tile-transposed node-per-lane layout (stage_lane.cuh), each
+//     node's slots sorted by gather row, and idxs, the same indices as 16-bit
+//     offsets from each node's own row,
 //   * PT:        the pointwise records [node][kPointStride].
 // Slots j >= nnbr get zero weights and gather the node's own row; nodes past n in
 // the last 32-node tile of Wl / idxl get zero weights and gather row pid0.  An
@@ -76,17 +77,25 @@ __global__ void pack_stencils_kernel(const T* __restrict__ Dx, const T* __restri
         }
         idxp[(i * 8 + k) * 4 + m] = p;
     }
-    const long b = i / kLaneTile, tt = i % kLaneTile;
-#pragma unroll
-    for (int op = 0; op < 4; ++op) {
-        const long unit = ((b * kSlots + j) * U + op / per_unit) * kLaneTile + tt;
-        Wl[unit * per_unit + op % per_unit] = w[op];
+    // node-per-lane layout: the node's slots by ascending gather row (ties in slot order)
+    int jl = j;
+    if (i < n && j < nnbr) {
+        const int own = idx_raw[cl.dm(i, j)];
+        jl = 0;
+        for (int o = 0; o < nnbr; ++o) {
+            const int q = idx_raw[cl.dm(i, o)];
+            jl += q < own || (q == own && o < j);
+        }
     }
-    idxl[(b * kSlots + j) * kLaneTile + tt] = p;
+    const long b = i / kLaneTile, tt = i % kLaneTile;
+    const long e = (b * kSlots + jl) * kLaneTile + tt;
+#pragma unroll
+    for (int op = 0; op < 4; ++op) Wl[4 * e + op] = w[op];
+    idxl[e] = p;
     // 16-bit offset from the node's own row (past n: from row n - 1 + pid0, offset 0)
     const int off = i < n ? p - ((int)i + pid0) : 0;
     if (off < -32768 || off > 32767) atomicOr(wide, 1);
-    idxs[(b * kSlots + j) * kLaneTile + tt] = (short)off;
+    idxs[e] = (short)off;
 }
 
 // One thread per node.
@@ -168,7 +177,7 @@ int pack_static_device(const CallerLayout& cl, int n, int rows, int pid0, int nn
     constexpr int per_unit = 16 / (int)sizeof(T);
     if ((e = cudaMalloc(&out.W, (size_t)n * kSlotChunks * U * 8 * per_unit * sizeof(T))) ||
         (e = cudaMalloc(&out.idx, (size_t)n * kSlots * sizeof(int))) ||
-        (e = cudaMalloc(&out.Wl, (size_t)npad * kSlots * U * per_unit * sizeof(T))) ||
+        (e = cudaMalloc(&out.Wl, (size_t)npad * kSlots * 4 * sizeof(T))) ||
         (e = cudaMalloc(&out.idxl, (size_t)npad * kSlots * sizeof(int))) ||
         (e = cudaMalloc(&out.idxs, (size_t)npad * kSlots * sizeof(short))) ||
         (e = cudaMalloc(&out.PT, (size_t)n * kPointStride * sizeof(T))))

@@ -57,7 +57,7 @@ struct alignas(16) ReqDesc {   // device table entry of an admitted request
     const uint4* W;      // grid: packed weights
     const int4* idx;     // grid: packed stencil indices
     const double* PT;    // grid: pointwise records
-    const uint4* Wl;     // grid: tile-transposed weights (node-per-lane split)
+    const double* Wl;    // grid: tile-transposed weights (node-per-lane split)
     const int* idxl;     // grid: tile-transposed stencil indices
     int n;               // nodes
     int nnbr;            // stencil slots in use (slot 31 of 31-neighbour stencils is padding)
@@ -102,9 +102,9 @@ __device__ __forceinline__ unsigned long long globaltimer() {
 }
 
 __device__ __forceinline__ void load_row_cg(const double* p, double (&v)[4]) {
-    const double2 a = __ldcg(reinterpret_cast<const double2*>(p));
-    const double2 b = __ldcg(reinterpret_cast<const double2*>(p) + 1);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+    asm volatile("ld.global.cg.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+                 : "l"(p));
 }
 
 // One warp, 16 nodes [base, base + 16) of one member and one stage, two lanes per
@@ -164,7 +164,7 @@ __device__ void serve_lanes(const ReqDesc& r, int stage, long base, long end, lo
     const long tile = i / kLaneTile;
     const int t = (int)(i % kLaneTile);
     const int* ip = r.idxl + (tile * kSlots + sub) * kLaneTile + t;
-    const uint4* wp = r.Wl + (tile * kSlots + sub) * 2 * kLaneTile + t;
+    const double* wp = r.Wl + ((tile * kSlots + sub) * kLaneTile + t) * 4;
     double acc[MB][16];
 #pragma unroll
     for (int m = 0; m < MB; ++m)
@@ -176,7 +176,7 @@ __device__ void serve_lanes(const ReqDesc& r, int stage, long base, long end, lo
         if (jj == kSlots / kSrvLpn - 1 && jj * kSrvLpn + sub >= r.nnbr) continue;
         const int p = lane::ld_stream(ip + jj * kSrvLpn * kLaneTile);
         double w[4];
-        lane::weights(wp + jj * kSrvLpn * 2 * kLaneTile, w);
+        lane::weights(wp + jj * kSrvLpn * kLaneTile * 4, lane::l2_normal(), w);
 #pragma unroll
         for (int m = 0; m < MB; ++m) {
             double kv[4];
@@ -525,7 +525,7 @@ struct Server {
         d.W = reinterpret_cast<const uint4*>(G.W);
         d.idx = reinterpret_cast<const int4*>(G.idx);
         d.PT = reinterpret_cast<const double*>(G.PT);
-        d.Wl = reinterpret_cast<const uint4*>(G.Wl);
+        d.Wl = reinterpret_cast<const double*>(G.Wl);
         d.idxl = G.idxl;
         d.n = G.n;
         d.nnbr = G.nnbr;

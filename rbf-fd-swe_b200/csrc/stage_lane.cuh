@@ -3,17 +3,24 @@
 // Same stage semantics as stage_kernel.cuh (eval_RHS_swe plus the RK4 stage
 // combine, swe_code/main/rk4_rbffd_swe.c:30-186 and :285-353), with a work split
 // that needs little or no cross-lane reduction: each of a node's LPN lanes (1, 2
-// or 4) sums the slots j = sub, sub + LPN, ... of the node serially -- with
-// LPN = 1 that is the reference's own slot order -- and the LPN partial sums
-// meet in a butterfly of log2(LPN) shuffle steps.  Lane sub 0 of every node then
+// or 4) sums the slots j = sub, sub + LPN, ... of the node serially, in ascending
+// order of the neighbours' rows, and the LPN partial sums meet in a butterfly of
+// log2(LPN) shuffle steps.  Lane sub 0 of every node then
 // runs the pointwise part and the stage combine, so up to all 32 lanes of a warp
 // are busy in the epilogue.
 //
 // The stencil weights and indices live in a second, tile-transposed copy
 // (pack_stencils_kernel in pack.cuh): per 32-node tile, slot-major, node-minor,
-// so one slot's weights of a warp's nodes are one contiguous 512-byte (FP64:
-// two) or 16-byte-per-lane (FP32) row and one slot's indices a contiguous
-// 128-byte row.  Weights and indices are streamed with L1 no-allocate loads; the
+// so one slot's weights of a warp's nodes are one contiguous 1024-byte (FP64) or
+// 512-byte (FP32) row and one slot's indices a contiguous 64- or 128-byte row.
+// Weights and FP64 state rows move as whole 32-byte sectors (256-bit loads), and
+// a node's slots are sorted by row: the L1 data pipe is what the kernel spends
+// most on when the data is in L2, and with sorted slots the lanes of a warp gather
+// neighbouring rows (N=40962, reverse Cuthill-McKee order: a 4-lane pass of a FP64
+// gather touches 19 of 32 lines against 24 in slot order).  N=40962 FP64: 10.2 us
+// per stage with 128-bit loads, 8.7 with 256-bit loads, 8.2 with sorted slots;
+// N=10242 5.1 / 4.1 / 4.1; N=655362 134.3 / 133.2 / 133.0.
+// Weights and indices are streamed with L1 no-allocate loads; the
 // neighbour gathers keep L1 to themselves.  One warp per unit of 32 / LPN nodes,
 // no persistent loop: the hardware scheduler balances the tail.  MINB (4 or 5)
 // is the register bound's CTAs per SM: 5 trades load depth for a grid that fits
@@ -31,13 +38,25 @@ constexpr int kLaneThreads = 128;
 constexpr int kLaneWarps = kLaneThreads / 32;
 constexpr int kLaneTile = 32;      // nodes per transposed tile of the packed arrays
 
+// Weights of more than 60 MB leave L2 (126 MB, shared with the state arrays, the pointwise
+// records and the indices) between two stages when every stage reads them in the same order.
+// From there on the stages alternate their direction and a quarter of the tiles is kept with
+// L2 priority.  Microseconds per stage in one order without / alternating with priorities:
+// FP64 N=40962 8.2 / 9.2 (weights 42 MB, below the line), N=60000 13.3 / 13.3, N=90000
+// 21.0 / 17.6, N=163842 36.4 / 30.3, N=655362 131.7 / 126.1; FP32 N=125000 14.8 / 14.4,
+// N=163842 18.4 / 14.9, N=655362 71.7 / 65.2.  Keeping 1/16, 1/8, 1/4, 1/2 or all of the
+// tiles: 31.3, 30.8, 30.3, 31.3 and 32.6 (FP64 N=163842).
+constexpr int kLaneKeep = 16;      // tiles of every 64 kept in L2
+inline bool lane_streams(long n, size_t fsize) { return n * kSlots * 4 * (long)fsize > 60L * 1000 * 1000; }
+
 template <typename T>
 struct LaneArgs {
     StageArgs<T> s;
-    const uint4* Wl;   // [tile][slot][unit][32 nodes] 16-byte units (FP64: (Dx,Dy), (Dz,L); FP32: all four)
+    const T* Wl;       // [tile][slot][32 nodes][4] weights (Dx, Dy, Dz, L)
     const int* idxl;   // [tile][slot][32 nodes] gather rows
     const short* idxs; // the same as 16-bit offsets from the node's own row (clamped to n - 1)
     int l2_prefetch;   // 1: bulk L2 prefetch of each warp's contiguous blocks at its start
+    int stream;        // 1: the weights do not fit in L2 (lane_streams)
     int nnbr;          // stencil slots in use: slots nnbr.. hold zero weights (a lane's last one is not read)
 };
 
@@ -53,28 +72,38 @@ __device__ __forceinline__ int ld_stream(const short* p) {
     asm volatile("ld.global.nc.L1::no_allocate.b16 %0, [%1];" : "=h"(v) : "l"(p));
     return v;
 }
-__device__ __forceinline__ double2 ld_stream(const double2* p) {
-    double2 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
-    return v;
+// the four weights (Dx, Dy, Dz, L) of one slot of one node
+__device__ __forceinline__ void weights(const double* p, uint64_t pol, double (&w)[4]) {
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f64 {%0, %1, %2, %3}, [%4], %5;"
+                 : "=d"(w[0]), "=d"(w[1]), "=d"(w[2]), "=d"(w[3])
+                 : "l"(p), "l"(pol));
 }
-__device__ __forceinline__ float4 ld_stream(const float4* p) {
-    float4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+__device__ __forceinline__ void weights(const float* p, uint64_t pol, float (&w)[4]) {
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+                 : "=f"(w[0]), "=f"(w[1]), "=f"(w[2]), "=f"(w[3])
+                 : "l"(p), "l"(pol));
+}
+// L2 priority of a tile's weights.  A patch whose weights do not fit in L2 reads them in
+// alternating directions (LaneArgs::stream) and keeps kLaneKeep of every 64 tiles with
+// priority, letting the others go first.
+__device__ __forceinline__ uint64_t l2_normal() {
+    uint64_t p;
+    asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ uint64_t l2_policy(int stream, long tile) {
+    uint64_t last, first;
+    asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(last));
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
+    return !stream ? l2_normal() : (tile & 63) < kLaneKeep ? last : first;
+}
+// one state row (u, v, w, h): a whole 32-byte sector in one load (FP64)
+__device__ __forceinline__ void state_row(const double* p, double (&v)[4]) {
+    asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
                  : "l"(p));
-    return v;
 }
-// the four weights (Dx, Dy, Dz, L) of one slot of node t; units of a slot are 32 x 16 bytes apart
-__device__ __forceinline__ void weights(const uint4* u, double (&w)[4]) {
-    const double2 a = ld_stream(reinterpret_cast<const double2*>(u));
-    const double2 b = ld_stream(reinterpret_cast<const double2*>(u + kLaneTile));
-    w[0] = a.x; w[1] = a.y; w[2] = b.x; w[3] = b.y;
-}
-__device__ __forceinline__ void weights(const uint4* u, float (&w)[4]) {
-    const float4 a = ld_stream(reinterpret_cast<const float4*>(u));
-    w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
-}
+__device__ __forceinline__ void state_row(const float* p, float (&v)[4]) { Quad<float>::load_row(p, v); }
 }  // namespace lane
 
 // I16: read the gather rows from the 16-bit offsets (half the index bytes); every
@@ -84,11 +113,12 @@ __global__ void __launch_bounds__(kLaneThreads, MINB) stage_lane_kernel(const La
     static_assert(LPN == 1 || LPN == 2 || LPN == 4, "1, 2 or 4 lanes per node");
     constexpr int kNpw = 32 / LPN;          // nodes per warp
     constexpr int kJpl = kSlots / LPN;      // slots per lane
-    constexpr int U = Quad<T>::kUnits;
     const StageArgs<T>& a = la.s;
     const int lane = threadIdx.x & 31;
     const int tl = lane % kNpw, sub = lane / kNpw;
-    const long node0 = ((long)blockIdx.x * kLaneWarps + (threadIdx.x >> 5)) * kNpw;
+    // odd stages run the tiles from the end: what the stage before read last is still in L2
+    const long bid = (MODE & 1) && la.stream ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+    const long node0 = (bid * kLaneWarps + (threadIdx.x >> 5)) * kNpw;
     const int nvalid = (int)min((long)kNpw, (long)a.n - node0);
     // With l2_prefetch, one lane requests the warp's contiguous blocks into L2 up
     // front, so that the loads below wait on L2 rather than DRAM: this warp's share
@@ -97,7 +127,7 @@ __global__ void __launch_bounds__(kLaneThreads, MINB) stage_lane_kernel(const La
     // patches the extra requests compete with the demand loads; on small ones it
     // gains little now that the gather rows are read before the wait, so the
     // init-time timing keeps it only where it is clearly faster.
-    constexpr uint32_t kTileW = kSlots * U * kLaneTile * 16, kTileI = kSlots * kLaneTile * (I16 ? 2 : 4);
+    constexpr uint32_t kTileW = kSlots * kLaneTile * 4 * sizeof(T), kTileI = kSlots * kLaneTile * (I16 ? 2 : 4);
     const bool pf = la.l2_prefetch != 0;
     if (pf && lane == 0 && nvalid > 0) {
         const long tb = node0 / kLaneTile;
@@ -140,7 +170,8 @@ __global__ void __launch_bounds__(kLaneThreads, MINB) stage_lane_kernel(const La
             prefetch_l2_bulk(a.D + 4 * node0, rows);
         }
     }
-    const uint4* wp = la.Wl + (tile * kSlots + sub) * U * kLaneTile + t;
+    const T* wp = la.Wl + ((tile * kSlots + sub) * kLaneTile + t) * 4;
+    const uint64_t pol = lane::l2_policy(la.stream, tile);
     T acc[16];
 #pragma unroll
     for (int q = 0; q < 16; ++q) acc[q] = T(0);
@@ -152,8 +183,8 @@ __global__ void __launch_bounds__(kLaneThreads, MINB) stage_lane_kernel(const La
         if (jj == kJpl - 1 && jj * LPN + sub >= la.nnbr) continue;
         const int p = kEarlyRows ? prow[kEarlyRows ? jj : 0] : row(jj);
         T w[4], kv[4];
-        lane::weights(wp + jj * LPN * U * kLaneTile, w);
-        Quad<T>::load_row(a.Kin + 4L * p, kv);
+        lane::weights(wp + jj * LPN * kLaneTile * 4, pol, w);
+        lane::state_row(a.Kin + 4L * p, kv);
 #pragma unroll
         for (int op = 0; op < 4; ++op)
 #pragma unroll
