@@ -75,3 +75,42 @@ def test_gpu_generated_input_steps_like_host_generated():
     rel = (np.abs(g - h).max(0) / scale).max()
     print(f"200 steps, GPU- vs host-weighted input: {rel:.2e}")
     assert rel <= 1e-8, rel
+
+
+def _spread(n, seed, cluster=0):
+    """Random unit vectors, `cluster` of them within 0.02 of one point."""
+    r = np.random.default_rng(seed)
+    X = r.standard_normal((n, 3))
+    X[:cluster] = np.array([0.3, -0.5, 0.8]) + 0.01 * r.standard_normal((cluster, 3))
+    return X / np.linalg.norm(X, axis=1, keepdims=True)
+
+
+@pytest.mark.parametrize("n,k,cluster", [(33, 32, 0), (40, 1, 0), (997, 17, 0), (1501, 31, 300), (2048, 32, 1000), (5000, 31, 0)])
+def test_stencils_of_uneven_nodes(n, k, cluster):
+    """Random and clustered nodes: too few or too many candidates within one cell edge send a
+    query from the warp search to the general one (nodes without distance ties)."""
+    X = _spread(n, n + k, cluster)
+    got = gen.stencils_gpu(X, k)
+    d = np.linalg.norm(X[:, None] - X[None], axis=2)
+    d[np.arange(n), np.arange(n)] = -1.0                        # self first
+    assert np.array_equal(got, np.argsort(d, axis=1, kind="stable")[:, :k])
+
+
+@pytest.mark.parametrize("k", [17, 25, 31, 32])
+def test_weights_of_other_stencil_sizes(k):
+    """Stencils narrower than the 32 places the solve holds, on nodes moved off the lattice."""
+    X = gen.icosahedral_nodes(3)
+    X = X + 0.005 * np.random.default_rng(k).standard_normal(X.shape)
+    X /= np.linalg.norm(X, axis=1, keepdims=True)
+    idx = gen.stencils(X, k)
+    for name, g, w in zip(("Dx", "Dy", "Dz", "L"), gen.rbffd_weights_gpu(X, idx), gen.rbffd_weights(X, idx, device="cpu")):
+        rel = np.abs(g - w).max() / np.abs(w).max()
+        assert rel <= 1e-8, (name, rel)
+
+
+def test_weights_of_coincident_nodes_are_refused():
+    X = gen.icosahedral_nodes(3)
+    idx = gen.stencils(X)
+    X[idx[100, 5]] = X[idx[100, 4]]
+    with pytest.raises(capi.SweError, match="singular"):
+        gen.rbffd_weights_gpu(X, idx)
