@@ -58,3 +58,43 @@ def test_patch_in_device_order_steps_like_oracle():
     finally:
         plain.finalize()
     assert rel_err(H, oracle.Port(m, "fp64").run(m.H_init, 20)).max() <= 1e-12
+
+
+def _tree(widths):
+    """Stencils of a tree whose levels hold `widths` nodes (at most 31 children a node),
+    numbered at random but for the root; unused slots name the node itself."""
+    n = sum(widths)
+    idx = np.repeat(np.arange(n, dtype=np.int32)[:, None], 32, 1)
+    first = np.cumsum([0] + list(widths))
+    for a, (w, v) in enumerate(zip(widths[:-1], widths[1:])):
+        for c in range(v):
+            idx[first[a] + c % w, 1 + c // w] = first[a + 1] + c
+    new = np.concatenate([[0], 1 + np.random.default_rng(n).permutation(n - 1)]).astype(np.int32)
+    out = np.empty_like(idx)
+    out[new] = new[idx]
+    return out
+
+
+class _Graph:
+    def __init__(self, idx):
+        self.idx, (self.N, self.Nnbr) = idx, idx.shape
+
+
+@pytest.mark.parametrize("widths", [(1,), (1, 1), (1, 31, 255, 257), (1, 31, 961, 4097, 5000), (1, 31, 961, 16384, 3)])
+def test_device_order_of_level_widths(widths):
+    """Levels around the cluster's warps, beyond what a warp keeps in shared memory, and of the
+    largest width."""
+    idx = _tree(widths)
+    assert np.array_equal(layout.rcm_mapping(_Graph(idx), device=True), levelset_mapping(idx))
+
+
+@pytest.mark.parametrize("case", ["wide", "apart", "index"])
+def test_device_order_refuses(case):
+    idx = _tree((1, 31, 961, 16385) if case == "wide" else (1, 31, 200))
+    if case == "apart":
+        idx[idx == 7] = 0
+        idx[7] = 7
+    if case == "index":
+        idx[100, 3] = len(idx)
+    with pytest.raises(capi.SweError, match={"wide": "more than 16384", "apart": "231 of 232", "index": "outside"}[case]):
+        layout.rcm_mapping(_Graph(idx), device=True)
