@@ -114,7 +114,10 @@ int swe_cuda_halo_setup(const int* send_rows, int n_send, const int* recv_rows, 
 int swe_cuda_halo_pack(int substep_id, void* send_buf);
 int swe_cuda_halo_unpack(int substep_id, const void* recv_buf);
 
-/* nsteps full RK4 steps (4 stages each) from a captured CUDA graph.
+/* nsteps full RK4 steps (4 stages each) from a captured CUDA graph, or, where
+ * swe_cuda_init found it faster (grids whose static data fits in the SMs' shared
+ * memory; no history output open; no kernel forced by swe_cuda_select_kernel), in
+ * one kernel that holds all SMs for the steps; the same bits either way.
  * Asynchronous; requires compute_pid_s == 0 and patch_size == compute_size
  * (no halo rows: a patch with halo rows steps by swe_cuda_rk_substep with
  * halo exchanges between substeps). */
@@ -357,13 +360,15 @@ int swe_srv_test_withhold(int request, int stage_index);
  * stream capture.  Calls share the array: calls that overlap on the GPU race
  * and must be serialised by the caller.  Kernels go to `stream` (a
  * cudaStream_t, NULL for the default stream); the call returns once they are
- * enqueued.  Every idx entry must lie in 0..n-1.  The kernels check each one
+ * enqueued.  Grids of a few thousand nodes or more whose static data fits in the
+ * SMs' shared memory step in one kernel that holds all SMs.  Every idx entry must lie in 0..n-1.  The kernels check each one
  * as they gather: an entry outside that range is never dereferenced (the node's
  * own row is read in its place, so that call's results are wrong) and the
  * first one is recorded.  A call with nsteps = 0 steps nothing: it waits for
  * `stream` and returns SWE_ERR_INDEX, naming the recorded (node, slot, value)
  * in swe_cuda_last_error(), if any earlier call met such an entry (clearing
- * the record), else SWE_OK. */
+ * the record), SWE_ERR_TIMEOUT if a bounded wait of an earlier call's kernel ran
+ * out, else SWE_OK. */
 #define SWE_NOALLOC_SCRATCH_BYTES (4u << 20)
 int swe_cuda_step_noalloc(int fsize, int n, int nnbr, double gh0, double dt, const int* idx,
                           const void* Dx, const void* Dy, const void* Dz, const void* L,

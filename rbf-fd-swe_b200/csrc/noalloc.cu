@@ -16,7 +16,9 @@
 //
 // The kernels are the fused stage kernel's math (stage_kernel.cuh) reading the
 // caller's row-major arrays directly instead of the packed device layout that
-// swe_cuda_init builds, so no packing buffer is needed either.
+// swe_cuda_init builds, so no packing buffer is needed either.  Grids of a few
+// thousand nodes or more whose static data fits in the SMs' shared memory run a
+// whole call in the resident kernel (resident.cuh), which lays it out there.
 //
 // The other entry points check every stencil index while packing it; here the
 // indices are read straight from the caller's device array, so the kernel
@@ -30,6 +32,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "resident.cuh"
 #include "stage_kernel.cuh"
 
 namespace swe {
@@ -43,6 +46,11 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocScratch
 // First out-of-range stencil index met by a kernel: {seen, node, slot, value}.
 // Zero at load; cleared by the nsteps = 0 call that reports it.
 static __device__ int g_noalloc_bad[4];
+
+// Arrival counter and abort word of the resident kernel, and its record of a wait that ran
+// out (cleared by the nsteps = 0 call that reports it).
+static __device__ __align__(128) unsigned g_noalloc_sync[res::kSyncWords];
+static __device__ int g_noalloc_failed;
 
 __device__ __forceinline__ int checked_neighbour(int v, int n, long node, int slot) {
     if ((unsigned)v < (unsigned)n) return v;
@@ -59,7 +67,14 @@ __device__ __forceinline__ int checked_neighbour(int v, int n, long node, int sl
 // host code the array's name is only a stand-in, so kernels get these.
 constexpr int kMaxDevices = 64;
 std::mutex g_setup_mu;
-void* g_scratch_addr[kMaxDevices] = {};
+struct StaticArrays {
+    void* scratch = nullptr;
+    unsigned* sync = nullptr;
+    int* failed = nullptr;
+    int sms = 0;
+    size_t smem = 0;          // shared memory a CTA may use
+};
+StaticArrays g_arrays[kMaxDevices];
 
 template <typename T>
 struct RowMajorArgs {
@@ -77,85 +92,123 @@ struct RowMajorArgs {
     double dt6;                    // dt/6
 };
 
+// One warp per 4 nodes, 8 lanes a node, slots j = k, k + 8, ... of lane k, as in
+// stage_kernel.  Everything static -- weights, rows, pointwise values -- is requested
+// before griddepcontrol.wait, so that a stage after the first starts on its gathers as
+// soon as the previous stage's states are visible, with its other operands on the way or
+// in place; the launches depend on one another programmatically (run_noalloc).
+// Bound by the chain of dependent L2 reads and the hand-over between launches: N=10242
+// FP64 6.4 us per stage, N=2562 3.1; 8.2 and 6.4 with plain launches and every load after
+// the launch.  Grids that fit the resident kernel take that from a few thousand nodes on
+// (resident_pays).
+constexpr int kRowThreads = 128, kRowWarps = kRowThreads / 32;
 template <typename T, int MODE>
-__global__ void __launch_bounds__(kStageThreads) rowmajor_stage_kernel(const RowMajorArgs<T> a) {
-    __shared__ __align__(16) T red[kStageWarps][4][16];
+__global__ void __launch_bounds__(kRowThreads, 4) rowmajor_stage_kernel(const RowMajorArgs<T> a) {
+    constexpr bool kHD = MODE == kStage1 || MODE == kStage2 || MODE == kStage3;
+    __shared__ __align__(16) T red[kRowWarps][4][16];
+    __shared__ __align__(16) T ep[kRowWarps][4][kPointStride + 12];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 3, k = lane & 7;
-    const long warps_total = (long)gridDim.x * kStageWarps;
-    for (long base = ((long)blockIdx.x * kStageWarps + warp) * 4; base < a.n; base += warps_total * 4) {
-        const long i = base + g;
-        const bool valid = i < a.n;
-        const long ii = valid ? i : (long)a.n - 1;
-        T acc[16];
+    const long i = ((long)blockIdx.x * kRowWarps + warp) * 4 + g;
+    const bool valid = i < a.n;
+    const long ii = valid ? i : (long)a.n - 1;
+    T* e = ep[warp][g];
+    T w[kSlotChunks][4];
+    int row[kSlotChunks];
 #pragma unroll
-        for (int t = 0; t < 16; ++t) acc[t] = T(0);
-#pragma unroll
-        for (int m = 0; m < kSlotChunks; ++m) {
-            const int j = 8 * m + k;           // same slot-to-lane split as stage_kernel
-            if (j < a.nnbr) {
-                const long e = ii * a.nnbr + j;
-                const T w[4] = {__ldg(a.Dx + e), __ldg(a.Dy + e), __ldg(a.Dz + e), __ldg(a.L + e)};
-                T kv[4];
-                Quad<T>::load_row(a.Kin + 4L * checked_neighbour(__ldg(a.idx + e), a.n, ii, j), kv);
-#pragma unroll
-                for (int op = 0; op < 4; ++op)
-#pragma unroll
-                    for (int fld = 0; fld < 4; ++fld) acc[op * 4 + fld] += w[op] * kv[fld];
-            }
+    for (int m = 0; m < kSlotChunks; ++m) {
+        const int j = 8 * m + k;
+        row[m] = -1;
+        if (j < a.nnbr) {
+            const long x = ii * a.nnbr + j;
+            row[m] = __ldg(a.idx + x);
+            w[m][0] = __ldg(a.Dx + x); w[m][1] = __ldg(a.Dy + x); w[m][2] = __ldg(a.Dz + x); w[m][3] = __ldg(a.L + x);
         }
-        T r0, r1;
-        reduce_scatter8(acc, k, r0, r1);
-        red[warp][g][2 * k] = r0;
-        red[warp][g][2 * k + 1] = r1;
-        __syncwarp();
-        if (k == 0 && valid) {
-            T s[16], pt[kPointStride], q[4], F[4];
-#pragma unroll
-            for (int t = 0; t < 16; ++t) s[t] = red[warp][g][t];
-            pt[PT_X] = a.x[i]; pt[PT_Y] = a.y[i]; pt[PT_Z] = a.z[i]; pt[PT_F] = a.f[i]; pt[PT_GHM] = a.ghm[i];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                pt[PT_PU + c] = a.pu[3 * i + c]; pt[PT_PV + c] = a.pv[3 * i + c];
-                pt[PT_PW + c] = a.pw[3 * i + c]; pt[PT_GG + c] = a.gg[3 * i + c];
-            }
-            Quad<T>::load_row(a.Kin + 4 * i, q);
-            pointwise_rhs(s, q, pt, a.gh0, F);
-            if (MODE == kStage0) {
-                T kn[4];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) kn[t] = Quad<T>::axpy(q[t], a.c, F[t]);
-                Quad<T>::store_row(a.D + 4 * i, F);
-                Quad<T>::store_row(a.Kout + 4 * i, kn);
-            } else if (MODE == kStage1 || MODE == kStage2) {
-                T h[4], d[4], kn[4];
-                Quad<T>::load_row_rw(a.H + 4 * i, h);
-                Quad<T>::load_row_rw(a.D + 4 * i, d);
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    d[t] = Quad<T>::axpy(d[t], T(2), F[t]);
-                    kn[t] = Quad<T>::axpy(h[t], a.c, F[t]);
-                }
-                Quad<T>::store_row(a.D + 4 * i, d);
-                Quad<T>::store_row(a.Kout + 4 * i, kn);
-            } else {
-                T h[4], d[4];
-                Quad<T>::load_row_rw(a.H + 4 * i, h);
-                Quad<T>::load_row_rw(a.D + 4 * i, d);
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    d[t] = Quad<T>::axpy(d[t], T(1), F[t]);
-                    h[t] = Quad<T>::update_h(h[t], a.dt6, d[t]);
-                }
-                Quad<T>::store_row(a.H + 4 * i, h);
-            }
-        }
-        __syncwarp();
     }
+    // pointwise values: lane k fetches the k-th scalar and the k-th vector
+    if (k < 5) e[k] = __ldg((k == 0 ? a.x : k == 1 ? a.y : k == 2 ? a.z : k == 3 ? a.f : a.ghm) + ii);
+    if (k < 4) {
+        const T* v = (k == 0 ? a.pu : k == 1 ? a.pv : k == 2 ? a.pw : a.gg) + 3 * ii;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) e[PT_PU + 3 * k + c] = __ldg(v + c);
+    }
+#pragma unroll
+    for (int m = 0; m < kSlotChunks; ++m)
+        if (8 * m + k < a.nnbr) row[m] = checked_neighbour(row[m], a.n, ii, 8 * m + k);
+    pdl_wait();
+    pdl_trigger();
+    T kv[kSlotChunks][4];
+#pragma unroll
+    for (int m = 0; m < kSlotChunks; ++m)
+        if (row[m] >= 0) Quad<T>::load_row(a.Kin + 4L * row[m], kv[m]);
+    // lanes 5-7: the own state and the H and D rows
+    if (k == 5 || (kHD && k > 5)) {
+        T r[4];
+        Quad<T>::load_row_rw((k == 5 ? a.Kin : k == 6 ? a.H : a.D) + 4 * ii, r);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) e[kPointStride + 4 * (k - 5) + x] = r[x];
+    }
+    T acc[16];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) acc[t] = T(0);
+#pragma unroll
+    for (int m = 0; m < kSlotChunks; ++m)
+        if (row[m] >= 0) {
+#pragma unroll
+            for (int op = 0; op < 4; ++op)
+#pragma unroll
+                for (int fld = 0; fld < 4; ++fld) acc[op * 4 + fld] += w[m][op] * kv[m][fld];
+        }
+    T r0, r1;
+    reduce_scatter8(acc, k, r0, r1);
+    red[warp][g][2 * k] = r0;
+    red[warp][g][2 * k + 1] = r1;
+    __syncwarp();
+    if (k != 0 || !valid) return;
+    T s[16], q[4], F[4];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) s[t] = red[warp][g][t];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) q[t] = e[kPointStride + t];
+    pointwise_rhs(s, q, e, a.gh0, F);
+    const T* h = e + kPointStride + 4;
+    const T* d = h + 4;
+    T out[4], dn[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        if (MODE == kStage0) {
+            dn[t] = F[t];
+            out[t] = Quad<T>::axpy(q[t], a.c, F[t]);
+        } else if (MODE != kStage3) {
+            dn[t] = Quad<T>::axpy(d[t], T(2), F[t]);
+            out[t] = Quad<T>::axpy(h[t], a.c, F[t]);
+        } else {
+            out[t] = Quad<T>::update_h(h[t], a.dt6, Quad<T>::axpy(d[t], T(1), F[t]));
+        }
+    }
+    if (MODE != kStage3) Quad<T>::store_row(a.D + 4 * i, dn);
+    Quad<T>::store_row((MODE == kStage3 ? a.H : a.Kout) + 4 * i, out);
 }
 
-// First call on the current device: look up the scratch array's address.
-int scratch_for_current_device(void** out) {
+// One stage on `stream`.  The call's first launch waits for everything before it on the
+// stream; the others may start while the stage before them ends, and read nothing that a
+// stage writes before their wait.
+template <typename T, int MODE>
+cudaError_t launch_stage(const RowMajorArgs<T>& a, bool first, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ceil_div(a.n, 4 * kRowWarps));
+    cfg.blockDim = dim3(kRowThreads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = first ? 0 : 1;
+    return cudaLaunchKernelEx(&cfg, rowmajor_stage_kernel<T, MODE>, a);
+}
+
+// First call on the current device: look up the static arrays' addresses.
+int arrays_of_current_device(StaticArrays& out) {
     int dev = 0;
     SWE_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= kMaxDevices) {
@@ -163,19 +216,103 @@ int scratch_for_current_device(void** out) {
         return SWE_ERR_ARG;
     }
     std::lock_guard<std::mutex> lock(g_setup_mu);
-    if (!g_scratch_addr[dev]) {
-        void* p = nullptr;
-        SWE_CUDA_TRY(cudaGetSymbolAddress(&p, g_noalloc_scratch));
-        g_scratch_addr[dev] = p;
+    StaticArrays& A = g_arrays[dev];
+    if (!A.scratch) {
+        void *scratch = nullptr, *sync = nullptr, *failed = nullptr;
+        SWE_CUDA_TRY(cudaGetSymbolAddress(&sync, g_noalloc_sync));
+        SWE_CUDA_TRY(cudaGetSymbolAddress(&failed, g_noalloc_failed));
+        SWE_CUDA_TRY(res::smem_limit(A.sms, A.smem));
+        SWE_CUDA_TRY(cudaGetSymbolAddress(&scratch, g_noalloc_scratch));
+        A.sync = (unsigned*)sync;
+        A.failed = (int*)failed;
+        A.scratch = scratch;
     }
-    *out = g_scratch_addr[dev];
+    out = A;
     return SWE_OK;
+}
+
+// Static data in the caller's row-major arrays (resident.cuh), indices checked.
+template <typename T>
+struct RowMajor {
+    static constexpr bool kNodeFast = false;    // a node's slots are contiguous
+    static constexpr bool kSmallRows = false;
+    const int* idx;
+    const T *Dx, *Dy, *Dz, *L;
+    const T *x, *y, *z, *f, *ghm;
+    const T *pu, *pv, *pw, *gg;
+    __device__ void weights(long i, int slot, int nnbr, T (&w)[4]) const {
+        const long e = i * nnbr + slot;
+        w[0] = __ldg(Dx + e); w[1] = __ldg(Dy + e); w[2] = __ldg(Dz + e); w[3] = __ldg(L + e);
+    }
+    __device__ int row(long i, int slot, int nnbr, int n) const {
+        return checked_neighbour(__ldg(idx + i * nnbr + slot), n, i, slot);
+    }
+    __device__ T point(long i, int k) const {
+        if (k >= PT_PU) {
+            const int v = (k - PT_PU) / 3, c = (k - PT_PU) % 3;
+            return __ldg((v == 0 ? pu : v == 1 ? pv : v == 2 ? pw : gg) + 3 * i + c);
+        }
+        return __ldg((k == 0 ? x : k == 1 ? y : k == 2 ? z : k == 3 ? f : ghm) + i);
+    }
+};
+
+// Whether the resident kernel's call is shorter than a launch per stage: its set-up, the
+// static data's way into shared memory, takes about 15 us.  us per call, stage launches /
+// resident: 20 steps FP64 N=2562 249 / 256, N=5000 361 / 278, N=10242 530 / 321, N=22000
+// 923 / 486, FP32 N=2562 214 / 228, N=10242 328 / 254, N=40962 881 / 395; 2 steps FP64
+// N=2562 46 / 51, N=5000 55 / 53, FP32 N=10242 52 / 51; 1 step FP64 N=5000 38 / 41, N=10242
+// 49 / 44, FP32 N=10242 37 / 40, N=20000 49 / 44.
+inline bool resident_pays(int n, int nsteps, size_t fsize) {
+    const size_t bytes = (size_t)n * fsize;
+    return bytes >= 80000 || (bytes >= 40000 && nsteps >= 2);
+}
+
+// Whole calls in the resident kernel: false where the grid does not fit it.
+template <typename T>
+bool run_resident(const RowMajorArgs<T>& r, T* Ka, T* Kb, T dt, int nsteps, const StaticArrays& A, cudaStream_t stream,
+                  cudaError_t& e) {
+    int m = 0, ctas = 0, lpn = 4;
+    size_t smem = 0;
+    if (!res::split<T>(r.n, r.nnbr, 4, A.sms, A.smem, m, ctas, smem)) {
+        lpn = 2;
+        if (!res::split<T>(r.n, r.nnbr, 2, A.sms, A.smem, m, ctas, smem)) return false;
+    }
+    res::Args<T> a{};
+    a.n = r.n;
+    a.nnbr = r.nnbr;
+    a.m = m;
+    a.nsteps = nsteps;
+    a.H = r.H;
+    a.Ka = Ka;
+    a.Kb = Kb;
+    a.gh0 = r.gh0;
+    a.c01 = (T)(dt / 2.0);
+    a.c2 = dt;
+    a.dt6 = r.dt6;
+    a.counter = A.sync;
+    a.failed = A.failed;
+    const RowMajor<T> src{r.idx, r.Dx, r.Dy, r.Dz, r.L, r.x, r.y, r.z, r.f, r.ghm, r.pu, r.pv, r.pw, r.gg};
+    e = lpn == 4 ? res::launch<T, 4>(a, src, ctas, smem, stream) : res::launch<T, 2>(a, src, ctas, smem, stream);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {      // fewer SMs for this stream than the device has
+        cudaGetLastError();
+        return false;
+    }
+    count_launch();
+    return true;
 }
 
 // nsteps = 0: wait for the caller's stream, then report (and clear) the first
 // out-of-range stencil index any earlier call met.
 int report_bad_index(cudaStream_t stream) {
     SWE_CUDA_TRY(cudaStreamSynchronize(stream));
+    int failed = 0;
+    SWE_CUDA_TRY(cudaMemcpyFromSymbol(&failed, g_noalloc_failed, sizeof(failed)));
+    if (failed) {
+        failed = 0;
+        SWE_CUDA_TRY(cudaMemcpyToSymbol(g_noalloc_failed, &failed, sizeof(failed)));
+        set_error("swe_cuda_step_noalloc: a bounded wait of an earlier call's kernel ran out (calls that overlapped?)");
+        return SWE_ERR_TIMEOUT;
+    }
     int bad[4] = {0, 0, 0, 0};
     SWE_CUDA_TRY(cudaMemcpyFromSymbol(bad, g_noalloc_bad, sizeof(bad)));
     if (!bad[0]) return SWE_OK;
@@ -191,9 +328,9 @@ int run_noalloc(int n, int nnbr, double gh0, double dt, const int* idx, const vo
                 const void* Dz, const void* L, const void* x, const void* y, const void* z, const void* f,
                 const void* ghm, const void* pu, const void* pv, const void* pw, const void* gg, void* H,
                 int nsteps, cudaStream_t stream) {
-    void* scratch = nullptr;
-    SWE_TRY(scratch_for_current_device(&scratch));
-    T* Ka = reinterpret_cast<T*>(scratch);
+    StaticArrays A;
+    SWE_TRY(arrays_of_current_device(A));
+    T* Ka = reinterpret_cast<T*>(A.scratch);
     T* Kb = Ka + 4L * n;
     T* D = Kb + 4L * n;
     RowMajorArgs<T> a{};
@@ -208,18 +345,21 @@ int run_noalloc(int n, int nnbr, double gh0, double dt, const int* idx, const vo
     a.gh0 = (T)gh0;
     const T dtT = (T)dt;
     a.dt6 = (double)dtT / 6.0;
-    const int grid = ceil_div(n, 4 * kStageWarps);
+    cudaError_t e = cudaSuccess;
+    if (resident_pays(n, nsteps, sizeof(T)) && run_resident<T>(a, Ka, Kb, dtT, nsteps, A, stream, e)) {
+        SWE_CUDA_TRY(e);
+        return SWE_OK;
+    }
     for (int s = 0; s < nsteps; ++s) {
         a.Kin = a.H; a.Kout = Ka; a.c = (T)(dtT / 2.0);
-        rowmajor_stage_kernel<T, kStage0><<<grid, kStageThreads, 0, stream>>>(a);
+        SWE_CUDA_TRY((launch_stage<T, kStage0>(a, s == 0, stream)));
         a.Kin = Ka; a.Kout = Kb;
-        rowmajor_stage_kernel<T, kStage1><<<grid, kStageThreads, 0, stream>>>(a);
+        SWE_CUDA_TRY((launch_stage<T, kStage1>(a, false, stream)));
         a.Kin = Kb; a.Kout = Ka; a.c = dtT;
-        rowmajor_stage_kernel<T, kStage2><<<grid, kStageThreads, 0, stream>>>(a);
+        SWE_CUDA_TRY((launch_stage<T, kStage2>(a, false, stream)));
         a.Kin = Ka; a.Kout = nullptr;
-        rowmajor_stage_kernel<T, kStage3><<<grid, kStageThreads, 0, stream>>>(a);
+        SWE_CUDA_TRY((launch_stage<T, kStage3>(a, false, stream)));
         count_launch(4);
-        SWE_CUDA_TRY(cudaGetLastError());
     }
     return SWE_OK;
 }

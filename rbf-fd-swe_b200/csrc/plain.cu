@@ -19,6 +19,7 @@
 #include "stage_tma.cuh"
 #include "stage_lane.cuh"
 #include "pack.cuh"
+#include "resident.cuh"
 
 namespace swe {
 
@@ -125,6 +126,12 @@ struct Plain {
 
     size_t fbytes(long count) const { return (size_t)count * fsize; }
 
+    // resident multi-step kernel (resident.cuh): lanes per node, 0 where it is not in use
+    int res_lpn = 0, res_m = 0, res_ctas = 0, res_min_steps = 1;
+    size_t res_smem = 0;
+    unsigned* res_sync = nullptr;
+    int* res_failed = nullptr;      // pinned: a bounded wait ran out
+
     HistoryWriter hist;             // history output (swe_hist_open)
     long long steps_done = 0;       // completed RK4 steps since the last swe_cuda_set_state
 
@@ -144,6 +151,11 @@ struct Plain {
         if (err_host) cudaFreeHost(err_host);
         err_host = nullptr;
         err_pending = false;
+        if (res_sync) cudaFree(res_sync);
+        if (res_failed) cudaFreeHost(res_failed);
+        res_sync = nullptr;
+        res_failed = nullptr;
+        res_lpn = 0;
         W = PT = H = Ka = Kb = D = F = Kx = raw = Wl = nullptr;
         idx = nullptr;
         idxl = nullptr;
@@ -321,6 +333,50 @@ struct Plain {
         return SWE_OK;
     }
 
+    template <typename T, int LPN>
+    cudaError_t launch_resident_t(int nsteps) {
+        res::Args<T> a{};
+        a.n = n;
+        a.nnbr = nnbr;
+        a.m = res_m;
+        a.nsteps = nsteps;
+        a.H = reinterpret_cast<T*>(H);
+        a.Ka = reinterpret_cast<T*>(Ka);
+        a.Kb = reinterpret_cast<T*>(Kb);
+        a.gh0 = (T)gh0;
+        const T dtT = (T)dt;
+        a.c01 = (T)(dtT / 2.0);
+        a.c2 = dtT;
+        a.dt6 = (double)dtT / 6.0;
+        a.counter = res_sync;
+        a.failed = res_failed;
+        const T* wl = reinterpret_cast<const T*>(Wl);
+        const T* pt = reinterpret_cast<const T*>(PT);
+        if (idxs_fit) return res::launch<T, LPN>(a, res::Packed<T, true>{wl, idxl, idxs, pt}, res_ctas, res_smem, stream);
+        return res::launch<T, LPN>(a, res::Packed<T, false>{wl, idxl, idxs, pt}, res_ctas, res_smem, stream);
+    }
+    cudaError_t launch_resident(int nsteps) {
+        count_launch();
+        if (fsize == 8) return res_lpn == 4 ? launch_resident_t<double, 4>(nsteps) : launch_resident_t<double, 2>(nsteps);
+        return res_lpn == 4 ? launch_resident_t<float, 4>(nsteps) : launch_resident_t<float, 2>(nsteps);
+    }
+    // Splits the grid over the SMs for lpn lanes a node (fits: false where it does not).
+    int setup_resident(int lpn, bool& fits) {
+        int nsm = 0;
+        size_t most = 0;
+        SWE_CUDA_TRY(res::smem_limit(nsm, most));
+        fits = fsize == 8 ? res::split<double>(n, nnbr, lpn, nsm, most, res_m, res_ctas, res_smem)
+                          : res::split<float>(n, nnbr, lpn, nsm, most, res_m, res_ctas, res_smem);
+        res_lpn = fits ? lpn : 0;
+        if (!fits) return SWE_OK;
+        if (!res_sync) {
+            SWE_CUDA_TRY(cudaMalloc(&res_sync, res::kSyncWords * sizeof(unsigned)));
+            SWE_CUDA_TRY(cudaHostAlloc(&res_failed, sizeof(int), cudaHostAllocDefault));
+            *res_failed = 0;
+        }
+        return SWE_OK;
+    }
+
     int build_graph() {
         cudaGraph_t g;
         SWE_CUDA_TRY(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
@@ -405,6 +461,13 @@ static int upload_static(Plain& P, const void* x, const void* y, const void* z, 
 // back enqueue their copy first, so one synchronisation serves both).
 static int check_tma_err() {
     Plain& P = g_plain;
+    if (P.res_failed && P.res_lpn) {
+        SWE_CUDA_TRY(cudaStreamSynchronize(P.stream));
+        if (*(volatile int*)P.res_failed) {
+            set_error("resident step kernel: a bounded wait for another block ran out");
+            return SWE_ERR_TIMEOUT;
+        }
+    }
     // only the pipelined kernel writes the word: read it back (one more small copy before
     // the synchronisation) only after such a launch
     if (!P.err || !P.err_host || !P.err_pending) {
@@ -567,8 +630,6 @@ int swe_cuda_init(int fsize, int layout, int simd_length, int compute_size, int 
             us_c[c] = ms * 1e3f / 9.f;
         }
         count_launch(12 * kCand);
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
         // the pipelined and node-per-lane kernels keep their fastest shapes, also
         // when another kernel wins
         int bt = 0, bl = kLane0;
@@ -594,6 +655,60 @@ int swe_cuda_init(int fsize, int layout, int simd_length, int compute_size, int 
             if (P.tune_us[k] < P.tune_us[best]) best = k;
         P.kernel_choice = best;
         SWE_TRY(check_tma_err());
+        // Whole steps in the resident kernel where it is faster than four launches of the
+        // stage kernel, with the stage kernel's lanes per node (a step and its four substeps
+        // give the same bits): 2 or 4, whichever of those whose stage kernel is within 3 % of
+        // the best gives the faster steps.  us per stage, stage kernel / resident: FP64 N=2562
+        // 3.1 / 2.8, N=10242 4.1 / 3.6, N=20000 6.2 / 4.8; FP32 N=40962 5.1 / 4.2.  Loading
+        // the static data costs about 15 us a call: res_min_steps steps pay for it.
+        if (best == 2 && compute_pid_s == 0 && patch_size == compute_size) {
+            int shape = -1, lpn_best = 0;
+            float step_best = 3.92f * us_c[bl], setup_best = 0.f;      // faster by 2 % at least
+            for (int l = 1; l <= 2; ++l) {
+                int bs = -1;                                           // best stage kernel shape of 2^l lanes
+                for (int c = kLane0; c < kCand; ++c)
+                    if ((c - kLane0) % 3 == l && (bs < 0 || us_c[c] < us_c[bs])) {
+                        lane_shape(P, c - kLane0);
+                        if (!P.lane_pf) bs = c;
+                    }
+                if ((bl - kLane0) % 3 == l) bs = bl;
+                bool fits = false;
+                if (us_c[bs] > 1.03f * us_c[bl]) continue;
+                SWE_TRY(P.setup_resident(1 << l, fits));
+                if (!fits) continue;
+                float ms[2] = {0.f, 0.f};
+                if (P.launch_resident(2) != cudaSuccess) {             // not enough SMs at once here
+                    cudaGetLastError();
+                    continue;
+                }
+                for (int r = 0; r < 4; ++r) {              // 2 and 10 steps, the first pair to warm up
+                    SWE_CUDA_TRY(cudaEventRecord(e0, P.stream));
+                    SWE_CUDA_TRY(P.launch_resident(r & 1 ? 10 : 2));
+                    SWE_CUDA_TRY(cudaEventRecord(e1, P.stream));
+                    SWE_CUDA_TRY(cudaEventSynchronize(e1));
+                    SWE_CUDA_TRY(cudaEventElapsedTime(&ms[r & 1], e0, e1));
+                }
+                SWE_TRY(check_tma_err());
+                const float step = (ms[1] - ms[0]) * 1e3f / 8.f;
+                if (step < step_best) {
+                    step_best = step;
+                    setup_best = ms[0] * 1e3f - 2.f * step;
+                    shape = bs;
+                    lpn_best = 1 << l;
+                }
+            }
+            // these steps moved H off its initial zero
+            SWE_CUDA_TRY(cudaMemsetAsync(P.H, 0, srow, P.stream));
+            lane_shape(P, (shape >= 0 ? shape : bl) - kLane0);
+            P.res_lpn = 0;
+            if (shape >= 0) {
+                bool fits = false;
+                SWE_TRY(P.setup_resident(lpn_best, fits));
+                P.res_min_steps = std::max(1, (int)std::ceil(setup_best / (4.f * us_c[bl] - step_best)));
+            }
+        }
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
     }
     if ((st = P.build_graph()) != SWE_OK) return st;
     return SWE_OK;
@@ -674,11 +789,18 @@ int swe_cuda_step(int nsteps) {
         SWE_CUDA_TRY(cudaEventRecord(P.step_ev[0], P.stream));
     }
     if (P.use_tma()) P.err_pending = true;
-    for (int s = 0; s < nsteps; ++s) {
+    int s = 0;
+    if (P.res_lpn && !P.hist.active() && nsteps >= P.res_min_steps) {
+        constexpr int kMost = 1000;          // steps per launch: a kernel of tens of milliseconds
+        for (; s < nsteps; s += std::min(kMost, nsteps - s)) SWE_CUDA_TRY(P.launch_resident(std::min(kMost, nsteps - s)));
+        P.steps_done += nsteps;
+        s = nsteps;
+    }
+    for (; s < nsteps; ++s) {
         SWE_CUDA_TRY(cudaGraphLaunch(P.graph, P.stream));
+        count_launch(4);
         SWE_TRY(after_step());
     }
-    count_launch(4LL * nsteps);
     if (P.timing) {
         SWE_CUDA_TRY(cudaEventRecord(P.step_ev[1], P.stream));
         P.step_timed = true;
@@ -787,6 +909,7 @@ int swe_cuda_select_kernel(int which) {
     if (piped && !P.tma_ok) { set_error("swe_cuda_select_kernel: the pipelined kernel is not set up"); return SWE_ERR_STATE; }
     SWE_CUDA_TRY(cudaStreamSynchronize(P.stream));
     P.kernel_choice = piped ? 0 : (which == 1 ? 1 : 2);
+    P.res_lpn = 0;          // the chosen stage kernel runs whole steps too
     if (which == 2) P.tma_tile = 64;
     if (which == 3) P.tma_tile = 32;
     if (which == 4) P.tma_tile = 16;

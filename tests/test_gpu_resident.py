@@ -1,0 +1,37 @@
+"""Whole steps of the plain form (swe_cuda_step) in the kernel swe_cuda_init chose, resident
+or one launch per stage, on small and mid-sized grids of odd sizes: the bits of the same
+number of swe_cuda_rk_substep rounds, and the oracle's states."""
+import numpy as np
+import pytest
+
+import oracle
+from conftest import scaled_err
+from swe_b200 import capi, layout
+from test_zz_no_alloc import _spiral
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("prec,n,nnbr", [("fp64", 149, 31), ("fp64", 1193, 20), ("fp64", 9731, 28), ("fp64", 23681, 31),
+                                         ("fp64", 31000, 25), ("fp32", 1185, 31), ("fp32", 20001, 32), ("fp32", 40001, 31)])
+def test_steps_equal_substeps_bitwise_and_match_oracle(prec, n, nnbr):
+    m = _spiral(n, nnbr)
+    m = layout.reorder(m, layout.rcm_mapping(m))
+    H0 = m.H_init.astype(np.float64 if prec == "fp64" else np.float32)
+    p = capi.Plain()
+    try:
+        p.init_model(m, prec)
+        got = {}
+        for steps in (1, 30):                       # a single step and one of many
+            p.set_state(H0)
+            p.step(steps)
+            got[steps] = p.get_state().reshape(-1, 4)
+            p.set_state(H0)
+            for _ in range(steps):
+                for s in range(4):
+                    p.rk_substep(s)
+            assert np.array_equal(got[steps], p.get_state().reshape(-1, 4)), steps
+    finally:
+        p.finalize()
+    want = oracle.Port(m, prec).run(H0, 30)
+    assert scaled_err(got[30], want).max() <= (1e-12 if prec == "fp64" else 1e-4)

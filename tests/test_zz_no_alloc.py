@@ -106,3 +106,88 @@ def test_noalloc_rejects_sizes_beyond_its_static_scratch():
     st = lib.swe_cuda_step_noalloc(8, limit + 1, 31, 0.0, 1.0, *([dummy] * 15), 1, None)
     assert st == 1
     assert b"static scratch" in lib.swe_cuda_last_error()
+
+
+def _spiral(n, nnbr):
+    """A grid of any size: nodes on a spiral, stencils and weights from the library's generator."""
+    from swe_b200 import gen
+    t = np.arange(n) + 0.5
+    z = 1.0 - 2.0 * t / n
+    r = np.sqrt(1.0 - z * z)
+    X = np.stack([r * np.cos(np.pi * (1 + 5 ** 0.5) * t), r * np.sin(np.pi * (1 + 5 ** 0.5) * t), z], 1)
+    idx = gen.stencils_gpu(X, nnbr)
+    Dx, Dy, Dz, L = gen.rbffd_weights_gpu(X, idx)
+    H, ghm = gen.tc5_state(X, n)
+    P = np.eye(3)[None] - X[:, :, None] * X[:, None, :]
+    gg = np.stack([np.einsum("ij,ij->i", D, ghm[idx]) / gen.A_EARTH for D in (Dx, Dy, Dz)], 1)
+    return swe_input.to_model(swe_input.SweInput(
+        N=n, Nnbr=nnbr, a=gen.A_EARTH, gh0=gen.G * gen.H0, dt=100.0, gamma=-gen.GAMMA_COEF * float(n) ** -4,
+        x=X[:, 0].copy(), y=X[:, 1].copy(), z=X[:, 2].copy(), f=2 * gen.OMEGA * X[:, 2], ghm=ghm, p_u=P[:, 0].copy(),
+        p_v=P[:, 1].copy(), p_w=P[:, 2].copy(), gradghm=gg, Dx=Dx, Dy=Dy, Dz=Dz, L=L, idx1=idx + 1, H_init=H,
+        H_100=np.zeros_like(H)))
+
+
+def _call(m, prec, nsteps, H, stream, t):
+    lib = _bind()
+    st = lib.swe_cuda_step_noalloc(
+        8 if prec == "fp64" else 4, m.N, m.Nnbr, float(m.gh0), float(m.dt), t["idx"].data_ptr(),
+        *[t[k].data_ptr() for k in ("Dx", "Dy", "Dz", "L", "x", "y", "z", "f", "ghm", "p_u", "p_v", "p_w", "gradghm")],
+        H.data_ptr(), nsteps, stream)
+    assert st == 0, lib.swe_cuda_last_error()
+
+
+def _device_arrays(m, prec):
+    import torch
+    dt = np.float64 if prec == "fp64" else np.float32
+    t = {k: torch.from_numpy(np.ascontiguousarray(getattr(m, k), dtype=dt)).cuda() for k in
+         ("Dx", "Dy", "Dz", "L", "x", "y", "z", "f", "ghm", "p_u", "p_v", "p_w", "gradghm")}
+    t["idx"] = torch.from_numpy(np.ascontiguousarray(m.idx, dtype=np.int32)).cuda()
+    return t
+
+
+# (nodes, neighbours): below and above the resident kernel's first size, nodes per block at and
+# around multiples of 8, its 512- and 640-thread shapes with 4 and 2 lanes a node, the largest
+# grids its shared memory holds and the first ones past it
+@pytest.mark.parametrize("prec,n,nnbr", [
+    ("fp64", 4999, 31), ("fp64", 5921, 17), ("fp64", 11840, 31), ("fp64", 18944, 32), ("fp64", 18945, 31),
+    ("fp64", 23681, 28), ("fp64", 27232, 31), ("fp64", 27233, 32), ("fp32", 10001, 31), ("fp32", 18945, 32),
+    ("fp32", 37889, 25), ("fp32", 47360, 31), ("fp32", 47361, 31)])
+def test_noalloc_sizes_match_oracle_steps(prec, n, nnbr):
+    import oracle
+    import torch
+
+    m = _spiral(n, nnbr)
+    t = _device_arrays(m, prec)
+    dt = np.float64 if prec == "fp64" else np.float32
+    buf = torch.empty(4 * n + 2, dtype=torch.float64 if prec == "fp64" else torch.float32, device="cuda")
+    for off in ((0, 2) if prec == "fp64" else (0,)):          # FP64: H 32- and 16-byte aligned
+        H = buf[off:off + 4 * n].view(n, 4)
+        H.copy_(torch.from_numpy(m.H_init.astype(dt)))
+        _call(m, prec, 3, H, torch.cuda.current_stream().cuda_stream, t)
+        want = oracle.Port(m, prec).run(m.H_init.astype(dt), 3)
+        assert scaled_err(H.cpu().numpy(), want).max() <= (1e-12 if prec == "fp64" else 1e-4)
+
+
+@pytest.mark.parametrize("n", [2000, 10242])
+def test_noalloc_calls_can_be_captured(n):
+    """A call captured in a CUDA graph and replayed twice gives what two calls give (stage
+    launches at the smaller size, the resident kernel at the larger)."""
+    import torch
+
+    m = _spiral(n, 31)
+    t = _device_arrays(m, "fp64")
+    H0 = torch.from_numpy(m.H_init).cuda()
+    want = H0.clone()
+    for _ in range(2):
+        _call(m, "fp64", 3, want, torch.cuda.current_stream().cuda_stream, t)
+    H = H0.clone()
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        _call(m, "fp64", 3, H, torch.cuda.current_stream().cuda_stream, t)
+    assert torch.equal(H, H0)
+    g.replay()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(H, want)
+    del g
