@@ -92,7 +92,9 @@ struct DevCtl {          // device-resident control words the host sets by async
 
 constexpr int kThreads = kStageThreads;         // 8 warps x 4 nodes
 static_assert(sizeof(ReqDesc) % 16 == 0 && sizeof(ReqDesc) / 16 <= kStageThreads, "descriptor copy");
-constexpr unsigned long long kIdleNs = 20ull * 1000 * 1000;          // idle exit after 20 ms
+// an idle kernel gives the GPU back after 1 ms: a relaunch costs some ten microseconds, and
+// other work of the process waits for the SMs meanwhile
+constexpr unsigned long long kIdleNs = 1000ull * 1000;
 constexpr unsigned long long kDepNs = 10ull * 1000 * 1000 * 1000;    // default dependency wait limit 10 s
 
 __device__ __forceinline__ unsigned long long globaltimer() {
@@ -107,11 +109,25 @@ __device__ __forceinline__ void load_row_cg(const double* p, double (&v)[4]) {
                  : "l"(p));
 }
 
+// A neighbour's row of the stage state: an L1-cached load.  Rows change between stages of one
+// launch; the fence that ends the item's dependency wait drops what L1 held before, and a row
+// is not rewritten until every item that reads its present value has finished.
+__device__ __forceinline__ void load_row_l1(const double* p, double (&v)[4]) {
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+                 : "l"(p));
+}
+
 // One warp, 16 nodes [base, base + 16) of one member and one stage, two lanes per
 // node: the node-per-lane stage kernel's math and data movement (stage_lane.cuh),
 // with L2-coherent loads of everything the kernel itself writes (states change
 // between stages inside one launch).  Nodes at or past `end` belong to another
 // work item (or pad the last tile): they are computed on valid rows and not stored.
+// Bound by the latency of the gathers in flight (128 registers a thread).  A saturated mix of
+// 32 requests over four grids: 5.96e9 node-stages/s with a row per slot read in the loop, both
+// members finished by one lane and L2-only gathers, 6.60e9 now; work items of 1024 nodes
+// instead of 2048: 5.47e9, claiming more items while one waits for its neighbours: 6.65e9,
+// but a burst of 12 small requests 33-37 ms instead of 28.
 constexpr int kSrvLpn = 2, kSrvNpw = 32 / kSrvLpn;
 constexpr int kSrvMB = 2;   // members per work item: each weight and index is loaded once for them
 static_assert(kSrvMB == 2, "serve_kernel dispatches blocks of one or two members");
@@ -165,6 +181,11 @@ __device__ void serve_lanes(const ReqDesc& r, int stage, long base, long end, lo
     const int t = (int)(i % kLaneTile);
     const int* ip = r.idxl + (tile * kSlots + sub) * kLaneTile + t;
     const double* wp = r.Wl + ((tile * kSlots + sub) * kLaneTile + t) * 4;
+    // the lane's rows at once: a row read in the slot loop puts its latency in front of every
+    // gather
+    int prow[kSlots / kSrvLpn];
+#pragma unroll
+    for (int jj = 0; jj < kSlots / kSrvLpn; ++jj) prow[jj] = lane::ld_stream(ip + jj * kSrvLpn * kLaneTile);
     double acc[MB][16];
 #pragma unroll
     for (int m = 0; m < MB; ++m)
@@ -174,29 +195,31 @@ __device__ void serve_lanes(const ReqDesc& r, int stage, long base, long end, lo
     for (int jj = 0; jj < kSlots / kSrvLpn; ++jj) {
         // a padding slot (zero weights) in a lane's last iteration moves no bytes
         if (jj == kSlots / kSrvLpn - 1 && jj * kSrvLpn + sub >= r.nnbr) continue;
-        const int p = lane::ld_stream(ip + jj * kSrvLpn * kLaneTile);
+        const int p = prow[jj];
         double w[4];
         lane::weights(wp + jj * kSrvLpn * kLaneTile * 4, lane::l2_normal(), w);
 #pragma unroll
         for (int m = 0; m < MB; ++m) {
             double kv[4];
-            load_row_cg(Kin + m * moff + 4L * p, kv);
+            load_row_l1(Kin + m * moff + 4L * p, kv);
 #pragma unroll
             for (int op = 0; op < 4; ++op)
 #pragma unroll
                 for (int f = 0; f < 4; ++f) acc[m][op * 4 + f] += w[op] * kv[f];
         }
     }
+    // each lane of a node's pair finishes one member: it adds the other lane's half of that
+    // member's sums (one member: the first lane)
+    static_assert(kSrvLpn == 2 && MB <= kSrvLpn, "a lane per member");
+    const int m = MB == 1 ? 0 : sub;
+    double sum[16];
 #pragma unroll
-    for (int m = 0; m < MB; ++m)
-#pragma unroll
-        for (int o = kSrvNpw; o < 32; o <<= 1)
-#pragma unroll
-            for (int q = 0; q < 16; ++q) acc[m][q] += __shfl_xor_sync(0xffffffffu, acc[m][q], o);
-    if (sub != 0 || i >= end) return;
-#pragma unroll
-    for (int m = 0; m < MB; ++m)
-        serve_epilogue(r, stage, i, acc[m], Hm + m * moff, Kin + m * moff, Kout + m * moff, Dm + m * moff);
+    for (int q = 0; q < 16; ++q) {
+        const double mine = m ? acc[MB - 1][q] : acc[0][q], other = m ? acc[0][q] : acc[MB - 1][q];
+        sum[q] = mine + __shfl_xor_sync(0xffffffffu, other, kSrvNpw);
+    }
+    if (sub >= MB || i >= end) return;
+    serve_epilogue(r, stage, i, sum, Hm + m * moff, Kin + m * moff, Kout + m * moff, Dm + m * moff);
 }
 
 // Exit is collective: the first CTA that has found the queue empty for kIdleNs
@@ -300,9 +323,9 @@ serve_kernel(Shared* ctl, const DevCtl* dctl, const Item* __restrict__ ring, lon
                     serve_lanes<1>(r, stage, base, end, moff, r.H + off, r.Ka + off, r.Kb + off, r.D + off, lane);
             }
         }
-        __threadfence();
         __syncthreads();
         if (threadIdx.x == 0) {
+            __threadfence();     // every thread's stores, ordered before this by the barrier
             // this chunk of these members has completed stage index q
             for (int m = 0; m < mb; ++m)
                 *(volatile int*)(r.cdone + (long)(it.member + m) * r.nchunks + it.chunk) = it.q + 1;
@@ -685,7 +708,7 @@ struct Server {
             if (!any) break;
         }
         if (appended) publish();
-        const bool work = tail > (long long)ctl->progress || !active.empty();
+        const bool work = !active.empty();       // (retired requests have no items left)
         if (ctl->error) return;                  // handled by the next pass
         const bool was_running = kernel_running();
         if (work && !was_running) launch_kernel();
