@@ -421,13 +421,24 @@ struct Ensemble {
     void launch_v(int mode) {
         using C = EnsCfg<T, MPC, PREC>;
         const EnsArgs a = args(mode, T, MPC);
-        const int grid = std::min(a.units, nsm);
+        // programmatic dependent launch: as the CTAs of a stage end, those of the next set up
+        // their barriers and tensor memory and start on the A images
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(std::min(a.units, nsm));
+        cfg.blockDim = dim3(C::kThreads);
+        cfg.dynamicSmemBytes = C::kSmem;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
         switch (mode) {
-            case 0: ens_stage_kernel<T, MPC, kStage0, PREC><<<grid, C::kThreads, C::kSmem, stream>>>(a); break;
-            case 1: ens_stage_kernel<T, MPC, kStage1, PREC><<<grid, C::kThreads, C::kSmem, stream>>>(a); break;
-            case 2: ens_stage_kernel<T, MPC, kStage2, PREC><<<grid, C::kThreads, C::kSmem, stream>>>(a); break;
-            case 3: ens_stage_kernel<T, MPC, kStage3, PREC><<<grid, C::kThreads, C::kSmem, stream>>>(a); break;
-            default: ens_stage_kernel<T, MPC, kEvalOnly, PREC><<<grid, C::kThreads, C::kSmem, stream>>>(a); break;
+            case 0: cudaLaunchKernelEx(&cfg, ens_stage_kernel<T, MPC, kStage0, PREC>, a); break;
+            case 1: cudaLaunchKernelEx(&cfg, ens_stage_kernel<T, MPC, kStage1, PREC>, a); break;
+            case 2: cudaLaunchKernelEx(&cfg, ens_stage_kernel<T, MPC, kStage2, PREC>, a); break;
+            case 3: cudaLaunchKernelEx(&cfg, ens_stage_kernel<T, MPC, kStage3, PREC>, a); break;
+            default: cudaLaunchKernelEx(&cfg, ens_stage_kernel<T, MPC, kEvalOnly, PREC>, a); break;
         }
     }
 

@@ -165,9 +165,17 @@ struct Cursor {
     bool valid;
 };
 
+// The unit a CTA takes as its position u of the stage's sequence: stages 1 and 3 run it from
+// the end, so that what the stage before touched last is still in L2.
+template <int MODE>
+__device__ __forceinline__ int unit_at(const EnsArgs& a, int u) {
+    return MODE == kStage1 || MODE == kStage3 ? a.units - 1 - u : u;
+}
+
+template <int MODE>
 __device__ __forceinline__ void unit_range(const EnsArgs& a, int u, int halves, int& g0, int& g1) {
     if (u < a.units) {
-        const int tile = u / halves;
+        const int tile = unit_at<MODE>(a, u) / halves;
         g0 = __ldg(a.row_off + tile) / kEnsKc;
         g1 = __ldg(a.row_off + tile + 1) / kEnsKc;
     } else {
@@ -175,17 +183,19 @@ __device__ __forceinline__ void unit_range(const EnsArgs& a, int u, int halves, 
     }
 }
 
+template <int MODE>
 __device__ __forceinline__ Cursor first_cursor(const EnsArgs& a, int halves) {
     Cursor p;
     p.u = blockIdx.x;
     p.ti = 0;
     p.valid = p.u < a.units;
-    unit_range(a, p.u, halves, p.gc, p.gc_end);
+    unit_range<MODE>(a, p.u, halves, p.gc, p.gc_end);
     p.gc0 = p.gc;
-    unit_range(a, p.u + gridDim.x, halves, p.nx_gc, p.nx_end);
+    unit_range<MODE>(a, p.u + gridDim.x, halves, p.nx_gc, p.nx_end);
     return p;
 }
 
+template <int MODE>
 __device__ __forceinline__ Cursor next_cursor(Cursor p, const EnsArgs& a, int halves) {
     if (!p.valid) return p;
     if (++p.gc < p.gc_end) return p;
@@ -194,7 +204,7 @@ __device__ __forceinline__ Cursor next_cursor(Cursor p, const EnsArgs& a, int ha
     p.valid = p.u < a.units;
     p.gc = p.gc0 = p.nx_gc;
     p.gc_end = p.nx_end;
-    unit_range(a, p.u + gridDim.x, halves, p.nx_gc, p.nx_end);
+    unit_range<MODE>(a, p.u + gridDim.x, halves, p.nx_gc, p.nx_end);
     return p;
 }
 
@@ -234,16 +244,6 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
         abort_s = 0;
         tc::fence_mbar_init();
     }
-    // split FP16: the field maxima hand over from step to step without another launch --
-    // stage 0 copies the ones it reads (the previous stage 3's) to where stages 1-3 read
-    // them, and stage 2 clears the slot stage 3 fills.  No launch reads a slot that the
-    // same launch writes.
-    if constexpr (PREC == kFp16x3) {
-        if (blockIdx.x == 0 && threadIdx.x < 4) {
-            if constexpr (MODE == kStage0) a.bmax_pub[threadIdx.x] = a.bmax[threadIdx.x];
-            if constexpr (MODE == kStage2) a.bmax_next[threadIdx.x] = 0u;
-        }
-    }
     if (warp == C::kMmaWarp) {
         tc::tmem_alloc(&tmem_s, C::kTmemCols);
         tc::tmem_relinquish();
@@ -257,7 +257,17 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
         // =============================== converters ===============================
         // FP16 operands: this thread's two fields (f0, f0 + 1) and their scales
         float2 sc = make_float2(1.f, 1.f);
+        pdl_wait();                 // the gathers and the maxima come from the previous stage
+        pdl_trigger();
         if constexpr (PREC == kFp16x3) {
+            // the field maxima hand over from step to step without another launch -- stage 0
+            // copies the ones it reads (the previous stage 3's) to where stages 1-3 read
+            // them, and stage 2 clears the slot stage 3 fills.  No launch reads a slot that
+            // the same launch writes.
+            if (blockIdx.x == 0 && threadIdx.x < 4) {
+                if constexpr (MODE == kStage0) a.bmax_pub[threadIdx.x] = a.bmax[threadIdx.x];
+                if constexpr (MODE == kStage2) a.bmax_next[threadIdx.x] = 0u;
+            }
             const int f0 = typename Op::Thread(threadIdx.x).col() & 3;
             sc = make_float2(ens::fp16_field_scale(a.bmax, f0, false), ens::fp16_field_scale(a.bmax, f0 + 1, false));
         }
@@ -268,9 +278,9 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
         unsigned char* stg0 = smem + C::kStgOff;
         // chunk g's gathers are issued two steps ahead as async copies into staging
         // buffer g % 3; the centre row of a new unit is loaded into a register then too
-        ens::Cursor cur = ens::first_cursor(a, halves);
-        ens::Cursor c1 = ens::next_cursor(cur, a, halves);
-        ens::Cursor c2 = ens::next_cursor(c1, a, halves);
+        ens::Cursor cur = ens::first_cursor<MODE>(a, halves);
+        ens::Cursor c1 = ens::next_cursor<MODE>(cur, a, halves);
+        ens::Cursor c2 = ens::next_cursor<MODE>(c1, a, halves);
         typename Op::Fetch f2, f3;     // indices of chunks g + 2 and g + 3
         using Cen = typename Op::Cen;
         Cen cen0{}, cen1{}, cen2{};    // centres of chunks g, g+1, g+2
@@ -278,8 +288,8 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
         auto issue = [&](const ens::Cursor& p, const typename Op::Fetch& f, int slot, Cen prev) {
             Cen c = prev;
             if (p.valid) {
-                const int tile = p.u / halves;
-                const long col = (long)(p.u % halves) * C::kN + th.col();
+                const int unit = ens::unit_at<MODE>(a, p.u), tile = unit / halves;
+                const long col = (long)(unit % halves) * C::kN + th.col();
                 Op::stage_issue(stg0 + slot * Op::kStgBytes, ct, a.Kin, a.mf, col, f);
                 if (p.gc == p.gc0) c = Op::load_cen(a.Kin + (long)__ldg(a.centre + tile) * a.mf + col);
             }
@@ -298,7 +308,7 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
         while (cur.valid) {
             // chunk g + 2's gathers, chunk g + 3's indices
             cen2 = issue(c2, f2, (g + 2) % 3, cen1);
-            const ens::Cursor c3 = ens::next_cursor(c2, a, halves);
+            const ens::Cursor c3 = ens::next_cursor<MODE>(c2, a, halves);
             if (c3.valid) Op::fetch_idx(a.rows, c3.gc, th, f3);
             asm volatile("cp.async.wait_group 2;" ::: "memory");
             const int s = g % C::kStages;
@@ -327,7 +337,7 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
                 const int ab = it & 1;
                 if (!ens::wait(&acce_bar[ab], ((it >> 1) & 1) ^ 1, abort_v, a.err, 4)) { ok = false; break; }
                 tc::fence_after_sync();
-                const int tile = u / halves;
+                const int tile = ens::unit_at<MODE>(a, u) / halves;
                 const int gc0 = __ldg(a.row_off + tile) / kEnsKc, gc1 = __ldg(a.row_off + tile + 1) / kEnsKc;
                 const uint32_t d = tmem + ab * C::kN;
                 for (int gc = gc0; gc < gc1; ++gc, ++g) {
@@ -355,8 +365,8 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
         {
             if (lane == 0) {
                 constexpr uint32_t kABytes = Op::kABytes;
-                ens::Cursor cur = ens::first_cursor(a, halves);
-                ens::Cursor pf = ens::next_cursor(ens::next_cursor(cur, a, halves), a, halves);
+                ens::Cursor cur = ens::first_cursor<MODE>(a, halves);
+                ens::Cursor pf = ens::next_cursor<MODE>(ens::next_cursor<MODE>(cur, a, halves), a, halves);
                 int g = 0;
                 while (cur.valid) {
                     const int s = g % C::kStages;
@@ -365,8 +375,8 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
                     tc::bulk_g2s(smem + s * C::kStageBytes, a.Aimg + (size_t)cur.gc * kABytes, kABytes, &afull_bar[s]);
                     if (pf.valid) prefetch_l2_bulk(a.Aimg + (size_t)pf.gc * kABytes, kABytes);
                     ++g;
-                    cur = ens::next_cursor(cur, a, halves);
-                    pf = ens::next_cursor(pf, a, halves);
+                    cur = ens::next_cursor<MODE>(cur, a, halves);
+                    pf = ens::next_cursor<MODE>(pf, a, halves);
                 }
                 // the copies of the last chunks land before the CTA ends, consumed or not
                 for (int k = g > C::kStages ? g - C::kStages : 0; k < g; ++k)
@@ -385,6 +395,7 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
         unsigned char* tbuf = smem + C::kStages * C::kStageBytes + kEnsEpiWarps * C::kXchWarpFloats * 4;
         const int members = a.members;
         const float c32 = (float)a.c;
+        pdl_wait();
         // FP16 operands: the state fields' inverse scales
         float binv[4] = {1.f, 1.f, 1.f, 1.f};
         if constexpr (PREC == kFp16x3) {
@@ -394,8 +405,8 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
         constexpr bool kHD = MODE == kStage1 || MODE == kStage2 || MODE == kStage3;
         // per-tile pointwise records (and, for split BF16, whose accumulator lacks the
         // add-back, the row sums and centre row): bulk copies into tbuf[it & 1]
-        auto issue_tile = [&](int u, int b) {
-            const int tile = u / halves;
+        auto issue_tile = [&](int pos, int b) {
+            const int u = ens::unit_at<MODE>(a, pos), tile = u / halves;
             const int nn = min(T, a.n - tile * T);
             unsigned char* tb = tbuf + b * C::kTileBuf;
             constexpr bool kAddBack = PREC == kBf16x3;
@@ -418,7 +429,6 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
         auto pair_member = [&](int pi) { return T == 32 ? (lane & 3) + 4 * pi : (lane + 32 * pi) & 7; };
         // streamed per-(node, member) operands of one chunk for this thread's pairs
         auto fetch = [&](int u, int ch, ens::EpiSet& o) {
-            if (u >= a.units) return;
             const int tile = u / halves;
             const int col0 = (u % halves) * C::kN;
 #pragma unroll
@@ -600,7 +610,7 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
                 pend = it + 1;
             }
 #pragma unroll 1
-            for (int c = 0; c < kCh; ++c) chunk(u, it, grp + 2 * c, sa);
+            for (int c = 0; c < kCh; ++c) chunk(ens::unit_at<MODE>(a, u), it, grp + 2 * c, sa);
             tc::fence_before_sync();
             __syncwarp();
             if (lane == 0) ens::mbar_arrive(&acce_bar[ab]);
