@@ -273,9 +273,10 @@ bool run_resident(const RowMajorArgs<T>& r, T* Ka, T* Kb, T dt, int nsteps, cons
                   cudaError_t& e) {
     int m = 0, ctas = 0, lpn = 4;
     size_t smem = 0;
-    if (!res::split<T>(r.n, r.nnbr, 4, A.sms, A.smem, m, ctas, smem)) {
+    bool stream_w = false;
+    if (!res::split<T>(r.n, r.nnbr, 4, A.sms, A.smem, false, m, ctas, smem, stream_w)) {
         lpn = 2;
-        if (!res::split<T>(r.n, r.nnbr, 2, A.sms, A.smem, m, ctas, smem)) return false;
+        if (!res::split<T>(r.n, r.nnbr, 2, A.sms, A.smem, false, m, ctas, smem, stream_w)) return false;
     }
     res::Args<T> a{};
     a.n = r.n;
@@ -292,7 +293,7 @@ bool run_resident(const RowMajorArgs<T>& r, T* Ka, T* Kb, T dt, int nsteps, cons
     a.counter = A.sync;
     a.failed = A.failed;
     const RowMajor<T> src{r.idx, r.Dx, r.Dy, r.Dz, r.L, r.x, r.y, r.z, r.f, r.ghm, r.pu, r.pv, r.pw, r.gg};
-    e = lpn == 4 ? res::launch<T, 4>(a, src, ctas, smem, stream) : res::launch<T, 2>(a, src, ctas, smem, stream);
+    e = lpn == 4 ? res::launch<T, 4>(a, src, ctas, smem, false, stream) : res::launch<T, 2>(a, src, ctas, smem, false, stream);
     if (e == cudaErrorCooperativeLaunchTooLarge) {      // fewer SMs for this stream than the device has
         cudaGetLastError();
         return false;

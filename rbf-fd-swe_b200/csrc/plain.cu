@@ -129,6 +129,7 @@ struct Plain {
     // resident multi-step kernel (resident.cuh): lanes per node, 0 where it is not in use
     int res_lpn = 0, res_m = 0, res_ctas = 0, res_min_steps = 1;
     size_t res_smem = 0;
+    bool res_stream = false;        // it streams part of the weights
     unsigned* res_sync = nullptr;
     int* res_failed = nullptr;      // pinned: a bounded wait ran out
 
@@ -352,8 +353,8 @@ struct Plain {
         a.failed = res_failed;
         const T* wl = reinterpret_cast<const T*>(Wl);
         const T* pt = reinterpret_cast<const T*>(PT);
-        if (idxs_fit) return res::launch<T, LPN>(a, res::Packed<T, true>{wl, idxl, idxs, pt}, res_ctas, res_smem, stream);
-        return res::launch<T, LPN>(a, res::Packed<T, false>{wl, idxl, idxs, pt}, res_ctas, res_smem, stream);
+        if (idxs_fit) return res::launch<T, LPN>(a, res::Packed<T, true>{wl, idxl, idxs, pt}, res_ctas, res_smem, res_stream, stream);
+        return res::launch<T, LPN>(a, res::Packed<T, false>{wl, idxl, idxs, pt}, res_ctas, res_smem, res_stream, stream);
     }
     cudaError_t launch_resident(int nsteps) {
         count_launch();
@@ -365,8 +366,8 @@ struct Plain {
         int nsm = 0;
         size_t most = 0;
         SWE_CUDA_TRY(res::smem_limit(nsm, most));
-        fits = fsize == 8 ? res::split<double>(n, nnbr, lpn, nsm, most, res_m, res_ctas, res_smem)
-                          : res::split<float>(n, nnbr, lpn, nsm, most, res_m, res_ctas, res_smem);
+        fits = fsize == 8 ? res::split<double>(n, nnbr, lpn, nsm, most, true, res_m, res_ctas, res_smem, res_stream)
+                          : res::split<float>(n, nnbr, lpn, nsm, most, true, res_m, res_ctas, res_smem, res_stream);
         res_lpn = fits ? lpn : 0;
         if (!fits) return SWE_OK;
         if (!res_sync) {
@@ -659,7 +660,7 @@ int swe_cuda_init(int fsize, int layout, int simd_length, int compute_size, int 
         // stage kernel, with the stage kernel's lanes per node (a step and its four substeps
         // give the same bits): 2 or 4, whichever of those whose stage kernel is within 3 % of
         // the best gives the faster steps.  us per stage, stage kernel / resident: FP64 N=2562
-        // 3.1 / 2.8, N=10242 4.1 / 3.6, N=20000 6.2 / 4.8; FP32 N=40962 5.1 / 4.2.  Loading
+        // 3.1 / 2.8, N=10242 4.1 / 3.6, N=20000 6.2 / 4.7, N=40962 8.2 / 7.2; FP32 N=40962 5.1 / 4.2.  Loading
         // the static data costs about 15 us a call: res_min_steps steps pay for it.
         if (best == 2 && compute_pid_s == 0 && patch_size == compute_size) {
             int shape = -1, lpn_best = 0;

@@ -16,11 +16,17 @@
 // visible.  Every wait is bounded: one that runs out raises an abort word that all CTAs
 // see in theirs, sets a flag for the host and ends the kernel.  The first wait of a launch
 // may be long, since other kernels may still hold some of the SMs.
+//
+// Weights that do not fit (FP64 from N = 27000 to 42600 on 148 SMs) are streamed from L2 in
+// every stage, see kStagePairs.  N=40962: 7.15 us per stage against 8.2 with a launch per
+// stage; 8.4 with plain loads of the nodes that do not fit, 7.9 with a copy per slot and
+// warp, 7.5 with two smaller buffers filled four times a stage.
 #pragma once
 
 #include <type_traits>
 
 #include "stage_lane.cuh"
+#include "tcgen05.cuh"
 
 namespace swe {
 namespace res {
@@ -60,6 +66,15 @@ struct Packed {
     }
     __device__ T point(long i, int f) const { return PT[i * kPointStride + f]; }
 };
+
+// Streamed weights (FP64, two lanes a node): the two warps of a 32-node tile hold the weights
+// of kHeldPairs slot pairs and stream the others through a buffer of kStagePairs pairs, filled
+// by one bulk copy twice a stage: the first batch while the stage before ends and the CTAs
+// meet, the second while the held pairs are summed.
+constexpr int kStagePairs = 7, kHeldPairs = 2;
+static_assert(2 * kStagePairs + kHeldPairs == kSlots / 2, "all slot pairs");
+constexpr int kBatchBytes = 2 * kStagePairs * kLaneTile * 4 * 8;
+constexpr uint32_t kCopyTries = 1u << 24;
 
 // A stage state row: a plain L1-cached load (never the non-coherent path, the rows change
 // between stages), one 32-byte sector.  FP64 rows of a caller's array (stage 0 reads H) may
@@ -140,15 +155,19 @@ __device__ __forceinline__ bool exchange(const Args<T>& a, unsigned stage, int* 
     return *s_ok != 0;
 }
 
-template <typename T, int LPN, int THREADS, class Src>
+template <typename T, int LPN, int THREADS, class Src, bool STREAM>
 __global__ void __launch_bounds__(THREADS, 1) steps_kernel(const Args<T> a, const Src src) {
     constexpr int kNpw = 32 / LPN;          // nodes per warp
     constexpr int kJpl = kSlots / LPN;      // slots per lane
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_ok;
-    const int nst = slots_of(a.nnbr, LPN);
+    static_assert(!STREAM || (sizeof(T) == 8 && LPN == 2), "streamed weights are FP64, two lanes a node");
+    __shared__ __align__(8) uint64_t s_bar[STREAM ? THREADS / 64 : 1];
+    const int nst = STREAM ? 2 * kHeldPairs : slots_of(a.nnbr, LPN);   // slots in shared memory
+    constexpr int kSlot0 = STREAM ? 2 * kStagePairs : 0;               // the first of them
     T* sw = reinterpret_cast<T*>(smem);
-    T* spt = sw + (long)nst * 4 * a.m;
+    T* sbuf = sw + (long)nst * 4 * a.m;                                // the tiles' buffers
+    T* spt = sbuf + (STREAM ? 2 * kStagePairs * 4 * a.m : 0);
     T* shd = spt + kPt * a.m;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tl = lane % kNpw, sub = lane / kNpw;
@@ -158,14 +177,14 @@ __global__ void __launch_bounds__(THREADS, 1) steps_kernel(const Args<T> a, cons
     for (int e = threadIdx.x; e < nst * a.m; e += blockDim.x) {
         const int slot = Src::kNodeFast ? e / a.m : e % nst, ln = Src::kNodeFast ? e % a.m : e / nst;
         T w[4] = {T(0), T(0), T(0), T(0)};
-        if (ln < cnt && slot < a.nnbr) src.weights(first + ln, slot, a.nnbr, w);
+        if (ln < cnt && kSlot0 + slot < a.nnbr) src.weights(first + ln, kSlot0 + slot, a.nnbr, w);
         put_weights(sw, a.m, slot, ln, w);
     }
     for (int e = threadIdx.x; e < kPt * cnt; e += blockDim.x) spt[e / cnt * a.m + e % cnt] = src.point(first + e % cnt, e / cnt);
     // this lane's node
     const int ln = warp * kNpw + tl;
     const bool valid = ln < cnt;
-    const bool active = warp * kNpw < cnt;                   // warp-uniform
+    const bool active = (STREAM ? warp & ~1 : warp) * kNpw < cnt;      // warp-uniform; streamed: both or none of a tile's
     const int lnc = min(ln, cnt - 1);
     const int own = (int)first + lnc;
     constexpr bool kPack = Src::kSmallRows && kJpl > 8;      // two 16-bit offsets a register
@@ -183,6 +202,38 @@ __global__ void __launch_bounds__(THREADS, 1) steps_kernel(const Args<T> a, cons
             }
         }
     }
+    // streamed weights: a batch of slot pairs from `pair0` on into the tile's buffer
+    T* buf = sbuf + (warp >> 1) * (kBatchBytes / 8);
+    uint64_t* bar = s_bar + (STREAM ? warp >> 1 : 0);
+    unsigned batches = 0;                  // batches waited for
+    bool pending = false;
+    auto fill = [&](int pair0) {
+        if constexpr (STREAM) {
+            // both warps have read the buffer, and their reads come before the copy
+            tc::fence_async_smem();
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp >> 1)) : "memory");
+            if ((warp & 1) == 0 && lane == 0) {
+                tc::mbar_arrive_expect_tx(bar, kBatchBytes);
+                tc::bulk_g2s(buf, src.Wl + 4 * src.at(first + warp * kNpw, 2 * pair0), kBatchBytes, bar);
+            }
+            pending = true;
+        }
+    };
+    auto filled = [&]() {
+        if constexpr (STREAM) {
+            if (!tc::mbar_wait_bounded(bar, batches & 1, kCopyTries)) {
+                *(volatile unsigned*)(a.counter + 32) = 1;
+                *(volatile int*)a.failed = 1;
+            }
+            ++batches;
+            pending = false;
+        }
+    };
+    if constexpr (STREAM) {
+        if ((warp & 1) == 0 && lane == 0) tc::mbar_init(bar, 1);
+        tc::fence_mbar_init();
+        if (active) fill(0);
+    }
     const bool wide_h = (reinterpret_cast<uintptr_t>(a.H) & 31) == 0;
     T q[4] = {};
     if (active) {
@@ -194,7 +245,7 @@ __global__ void __launch_bounds__(THREADS, 1) steps_kernel(const Args<T> a, cons
     __syncthreads();
     unsigned done = 0;
 
-    auto stage = [&](auto mode_c) {
+    auto stage = [&](auto mode_c, bool more) {
         constexpr int MODE = decltype(mode_c)::value;
         if (!active) return;
         const T* Kin = MODE == kStage0 ? a.H : MODE == kStage2 ? a.Kb : a.Ka;
@@ -209,31 +260,60 @@ __global__ void __launch_bounds__(THREADS, 1) steps_kernel(const Args<T> a, cons
         T acc[16];
 #pragma unroll
         for (int x = 0; x < 16; ++x) acc[x] = T(0);
-        constexpr int kChunk = 4;
+        // pairs (slots of this lane) [from, to), weights by get(pair, w)
+        auto sum = [&](auto from_c, auto to_c, auto get) {
+            constexpr int kFrom = decltype(from_c)::value, kTo = decltype(to_c)::value, kChunk = 4;
 #pragma unroll
-        for (int j0 = 0; j0 < kJpl; j0 += kChunk) {
-            if (j0 * LPN >= a.nnbr) break;
-            T kv[kChunk][4];
+            for (int j0 = kFrom; j0 < kTo; j0 += kChunk) {
+                if (j0 * LPN >= a.nnbr) break;
+                T kv[kChunk][4];
 #pragma unroll
-            for (int u = 0; u < kChunk; ++u) {
-                const int jj = j0 + u;
-                int p;
-                if constexpr (kPack) p = own + (jj & 1 ? rows[jj / 2] >> 16 : (int)(short)rows[jj / 2]);
-                else p = rows[jj];
-                load_state(Kin + 4L * p, wide, kv[u]);
+                for (int u = 0; u < kChunk; ++u) {
+                    const int jj = j0 + u;
+                    if (jj >= kTo) continue;
+                    int p;
+                    if constexpr (kPack) p = own + (jj & 1 ? rows[jj / 2] >> 16 : (int)(short)rows[jj / 2]);
+                    else p = rows[jj];
+                    load_state(Kin + 4L * p, wide, kv[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < kChunk; ++u) {
+                    if (j0 + u >= kTo) continue;
+                    // (slots at or past nnbr: the own row with zero weights)
+                    if (!STREAM && (j0 + u) * LPN >= nst) continue;
+                    T w[4];
+                    get(j0 + u, w);
+#pragma unroll
+                    for (int op = 0; op < 4; ++op)
+#pragma unroll
+                        for (int f = 0; f < 4; ++f) acc[op * 4 + f] += w[op] * kv[u][f];
+                }
             }
-#pragma unroll
-            for (int u = 0; u < kChunk; ++u) {
-                const int slot = (j0 + u) * LPN + sub;
-                // (slots at or past nnbr: the own row with zero weights)
-                if ((j0 + u) * LPN >= nst) continue;
-                T w[4];
-                get_weights(sw, m, slot, lnc, w);
-#pragma unroll
-                for (int op = 0; op < 4; ++op)
-#pragma unroll
-                    for (int f = 0; f < 4; ++f) acc[op * 4 + f] += w[op] * kv[u][f];
-            }
+        };
+        auto held = [&](int jj, T (&w)[4]) { get_weights(sw, m, jj * LPN + sub - kSlot0, lnc, w); };
+        if constexpr (STREAM) {
+            // a node's four weights lie together: lanes 4..7 of each eight read their second
+            // half first, so that a pass of 16-byte reads meets no bank twice
+            const bool swap = tl & 4;
+            int base = 0;
+            auto streamed = [&](int jj, T (&w)[4]) {
+                const double2* p = reinterpret_cast<const double2*>(buf + (((jj - base) * 2 + sub) * kLaneTile + (warp & 1) * kNpw + tl) * 4);
+                const double2 x = p[swap], y = p[!swap];
+                w[0] = swap ? y.x : x.x; w[1] = swap ? y.y : x.y;
+                w[2] = swap ? x.x : y.x; w[3] = swap ? x.y : y.y;
+            };
+            using std::integral_constant;
+            constexpr int kA = kStagePairs, kB = kStagePairs + kHeldPairs;
+            filled();
+            sum(integral_constant<int, 0>(), integral_constant<int, kA>(), streamed);
+            fill(kB);
+            sum(integral_constant<int, kA>(), integral_constant<int, kB>(), held);
+            filled();
+            base = kB;
+            sum(integral_constant<int, kB>(), integral_constant<int, kJpl>(), streamed);
+            if (more) fill(0);
+        } else {
+            sum(std::integral_constant<int, 0>(), std::integral_constant<int, kJpl>(), held);
         }
 #pragma unroll
         for (int o = kNpw; o < 32; o <<= 1)
@@ -263,30 +343,42 @@ __global__ void __launch_bounds__(THREADS, 1) steps_kernel(const Args<T> a, cons
     };
 
     for (int s = 0; s < a.nsteps; ++s) {
-        stage(std::integral_constant<int, kStage0>());
-        if (!exchange(a, ++done, &s_ok)) return;
-        stage(std::integral_constant<int, kStage1>());
-        if (!exchange(a, ++done, &s_ok)) return;
-        stage(std::integral_constant<int, kStage2>());
-        if (!exchange(a, ++done, &s_ok)) return;
-        stage(std::integral_constant<int, kStage3>());
-        if (s + 1 < a.nsteps && !exchange(a, ++done, &s_ok)) return;
+        const bool last = s + 1 == a.nsteps;
+        stage(std::integral_constant<int, kStage0>(), true);
+        if (!exchange(a, ++done, &s_ok)) break;
+        stage(std::integral_constant<int, kStage1>(), true);
+        if (!exchange(a, ++done, &s_ok)) break;
+        stage(std::integral_constant<int, kStage2>(), true);
+        if (!exchange(a, ++done, &s_ok)) break;
+        stage(std::integral_constant<int, kStage3>(), !last);
+        if (!last && !exchange(a, ++done, &s_ok)) break;
     }
+    if (pending) filled();                 // after an abort: no copy in flight when the block ends
 }
 
 // How a grid of n nodes is split over the SMs with lpn lanes a node: nodes per CTA (a multiple
-// of 8) and CTAs.  False where a CTA's nodes exceed its threads or smem_max bytes.
+// of 8) and CTAs, and whether the weights are streamed (only where Src allows it: `streams`).
+// False where a CTA's nodes exceed its threads or smem_max bytes.
 template <typename T>
-inline bool split(int n, int nnbr, int lpn, int sms, size_t smem_max, int& m, int& ctas, size_t& smem) {
+inline bool split(int n, int nnbr, int lpn, int sms, size_t smem_max, bool streams, int& m, int& ctas, size_t& smem,
+                  bool& stream) {
     m = ((n + sms - 1) / sms + 7) / 8 * 8;
-    ctas = (n + m - 1) / m;
     smem = m * ((kPt + 8) * sizeof(T) + slots_of(nnbr, lpn) * 4 * sizeof(T));
+    stream = false;
+    if (smem > smem_max && streams && sizeof(T) == 8 && lpn == 2) {
+        m = (m + kLaneTile - 1) / kLaneTile * kLaneTile;      // whole tiles
+        smem = m * ((kPt + 8) * sizeof(T) + 2 * (kStagePairs + kHeldPairs) * 4 * sizeof(T));
+        stream = true;
+    }
+    ctas = (n + m - 1) / m;
     return m * lpn <= kMost && smem <= smem_max;
 }
 
 template <typename T, int LPN, class Src>
-inline cudaError_t launch(const Args<T>& a, const Src& src, int ctas, size_t smem, cudaStream_t st) {
-    auto kernel = a.m * LPN <= kFew ? steps_kernel<T, LPN, kFew, Src> : steps_kernel<T, LPN, kMost, Src>;
+inline cudaError_t launch(const Args<T>& a, const Src& src, int ctas, size_t smem, bool stream, cudaStream_t st) {
+    auto kernel = a.m * LPN <= kFew ? steps_kernel<T, LPN, kFew, Src, false> : steps_kernel<T, LPN, kMost, Src, false>;
+    if constexpr (Src::kNodeFast && sizeof(T) == 8 && LPN == 2)
+        if (stream) kernel = steps_kernel<T, LPN, kMost, Src, true>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(a.counter, 0, kSyncWords * sizeof(unsigned), st);

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("prec,n,nnbr", [("fp64", 149, 31), ("fp64", 1193, 20), ("fp64", 9731, 28), ("fp64", 23681, 31),
-                                         ("fp64", 31000, 25), ("fp32", 1185, 31), ("fp32", 20001, 32), ("fp32", 40001, 31)])
+                                         ("fp64", 31000, 25), ("fp64", 35009, 31), ("fp64", 42600, 32), ("fp32", 1185, 31), ("fp32", 20001, 32), ("fp32", 40001, 31)])
 def test_steps_equal_substeps_bitwise_and_match_oracle(prec, n, nnbr):
     m = _spiral(n, nnbr)
     m = layout.reorder(m, layout.rcm_mapping(m))
