@@ -63,6 +63,8 @@ constexpr int kPointStride = 20;                      // per-node pointwise valu
 enum PointField { PT_X = 0, PT_Y, PT_Z, PT_F, PT_GHM, PT_PU, PT_PV = PT_PU + 3, PT_PW = PT_PV + 3,
                   PT_GG = PT_PW + 3 };
 
+constexpr int kPointFields = PT_GG + 3;               // values in use
+
 inline int ceil_div(long a, long b) { return (int)((a + b - 1) / b); }
 
 // Programmatic dependent launch.  The previous stage's writes are visible only

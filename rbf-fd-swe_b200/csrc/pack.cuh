@@ -11,7 +11,8 @@
 //   * Wl / idxl: the tile-transposed node-per-lane layout (stage_lane.cuh), each
 //     node's slots placed so that neighbouring lanes gather the same lines, and
 //     idxs, the same indices as 16-bit offsets from each node's own row,
-//   * PT:        the pointwise records [node][kPointStride].
+//   * PT:        the pointwise records [node][kPointStride], and PTl, the same
+//     values tile-transposed for the node-per-lane kernels.
 // Slots j >= nnbr get zero weights and gather the node's own row; nodes past n in
 // the last 32-node tile of Wl / idxl get zero weights and gather row pid0.  An
 // index outside [0, rows) is reported as the first offending (node, slot) in
@@ -38,9 +39,10 @@ struct PackedStatic {
     short* idxs = nullptr;  // the same as 16-bit offsets from the node's own row
     bool idxs_ok = false;   // every offset fits 16 bits
     T* PT = nullptr;      // pointwise records
+    T* PTl = nullptr;     // tile-transposed pointwise values
     void release() {
-        for (void* p : {(void*)W, (void*)idx, (void*)Wl, (void*)idxl, (void*)idxs, (void*)PT}) if (p) cudaFree(p);
-        W = nullptr; idx = nullptr; Wl = nullptr; idxl = nullptr; idxs = nullptr; PT = nullptr;
+        for (void* p : {(void*)W, (void*)idx, (void*)Wl, (void*)idxl, (void*)idxs, (void*)PT, (void*)PTl}) if (p) cudaFree(p);
+        W = nullptr; idx = nullptr; Wl = nullptr; idxl = nullptr; idxs = nullptr; PT = PTl = nullptr;
         idxs_ok = false;
     }
 };
@@ -165,17 +167,23 @@ __global__ void pack_lanes_kernel(const T* __restrict__ Dx, const T* __restrict_
     }
 }
 
-// One thread per node.
+// One thread per node (and per place of the last tile).
 template <typename T>
 __global__ void pack_points_kernel(const T* __restrict__ x, const T* __restrict__ y, const T* __restrict__ z,
                                    const T* __restrict__ f, const T* __restrict__ ghm, const T* __restrict__ pu,
                                    const T* __restrict__ pv, const T* __restrict__ pw, const T* __restrict__ gg,
-                                   CallerLayout cl, int n, T* __restrict__ PT) {
+                                   CallerLayout cl, int n, long npad, T* __restrict__ PT, T* __restrict__ PTl) {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= npad) return;
     T r[kPointStride];
 #pragma unroll
     for (int k = 0; k < kPointStride; ++k) r[k] = T(0);
+    T* l = PTl + i / kLaneTile * kPointFields * kLaneTile + i % kLaneTile;
+    if (i >= n) {                                    // past n in the last tile
+#pragma unroll
+        for (int k = 0; k < kPointFields; ++k) l[k * kLaneTile] = T(0);
+        return;
+    }
     r[PT_X] = x[i]; r[PT_Y] = y[i]; r[PT_Z] = z[i]; r[PT_F] = f[i]; r[PT_GHM] = ghm[i];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -184,6 +192,8 @@ __global__ void pack_points_kernel(const T* __restrict__ x, const T* __restrict_
     }
 #pragma unroll
     for (int k = 0; k < kPointStride; ++k) PT[i * kPointStride + k] = r[k];
+#pragma unroll
+    for (int k = 0; k < kPointFields; ++k) l[k * kLaneTile] = r[k];
 }
 
 namespace pack_detail {
@@ -247,7 +257,8 @@ int pack_static_device(const CallerLayout& cl, int n, int rows, int pid0, int nn
         (e = cudaMalloc(&out.Wl, (size_t)npad * kSlots * 4 * sizeof(T))) ||
         (e = cudaMalloc(&out.idxl, (size_t)npad * kSlots * sizeof(int))) ||
         (e = cudaMalloc(&out.idxs, (size_t)npad * kSlots * sizeof(short))) ||
-        (e = cudaMalloc(&out.PT, (size_t)n * kPointStride * sizeof(T))))
+        (e = cudaMalloc(&out.PT, (size_t)n * kPointStride * sizeof(T))) ||
+        (e = cudaMalloc(&out.PTl, (size_t)npad * kPointFields * sizeof(T))))
         return fail(e);
     if ((e = cudaMallocAsync(reinterpret_cast<void**>(&bad), sizeof(*bad), st))) return fail(e);
     owned.push_back(bad);
@@ -261,8 +272,8 @@ int pack_static_device(const CallerLayout& cl, int n, int rows, int pid0, int nn
                                                                               rows, pid0, out.W, out.idx, bad);
     pack_lanes_kernel<T><<<(unsigned)((groups + 7) / 8), 256, 0, st>>>(tDx, tDy, tDz, tL, tidx, cl, n, npad, nnbr, rows,
                                                                       pid0, out.Wl, out.idxl, out.idxs, wide);
-    pack_points_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(tx, ty, tz, tf, tghm, tpu, tpv, tpw, tgg, cl,
-                                                                      n, out.PT);
+    pack_points_kernel<T><<<(unsigned)((npad + 255) / 256), 256, 0, st>>>(tx, ty, tz, tf, tghm, tpu, tpv, tpw, tgg, cl,
+                                                                         n, npad, out.PT, out.PTl);
     count_launch(3);
     unsigned long long hb = ULLONG_MAX;
     int hw = 1;

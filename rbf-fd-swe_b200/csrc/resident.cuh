@@ -35,7 +35,7 @@ namespace res {
 // with FP64)
 constexpr int kFew = 512, kMost = 640;
 constexpr int kSyncWords = 64;         // counter and abort word, a line each
-constexpr int kPt = 17;                // pointwise values in use
+constexpr int kPt = kPointFields;
 constexpr unsigned long long kWaitNs = 2000000000ull, kFirstWaitNs = 60000000000ull;
 
 template <typename T>
@@ -58,13 +58,15 @@ struct Packed {
     const T* Wl;
     const int* idxl;
     const short* idxs;
-    const T* PT;
+    const T* PTl;
     __device__ static long at(long i, int slot) { return ((i / kLaneTile) * kSlots + slot) * kLaneTile + i % kLaneTile; }
     __device__ void weights(long i, int slot, int, T (&w)[4]) const { lane::weights(Wl + 4 * at(i, slot), lane::l2_normal(), w); }
     __device__ int row(long i, int slot, int, int) const {
         return I16 ? (int)i + lane::ld_stream(idxs + at(i, slot)) : lane::ld_stream(idxl + at(i, slot));
     }
-    __device__ T point(long i, int f) const { return PT[i * kPointStride + f]; }
+    __device__ T point(long i, int f) const {
+        return PTl[(i / kLaneTile * kPointFields + f) * kLaneTile + i % kLaneTile];
+    }
 };
 
 // Streamed weights (FP64, two lanes a node): the two warps of a 32-node tile hold the weights
@@ -339,7 +341,8 @@ __global__ void __launch_bounds__(THREADS, 1) steps_kernel(const Args<T> a, cons
                 sh[x * a.m] = q[x];
             }
         }
-        Quad<T>::store_row(Kout + 4L * own, q);
+        if (MODE != kStage3 || wide_h) lane::put_row(Kout + 4L * own, q);
+        else Quad<T>::store_row(Kout + 4L * own, q);
     };
 
     for (int s = 0; s < a.nsteps; ++s) {

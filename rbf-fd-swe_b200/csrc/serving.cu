@@ -56,7 +56,7 @@ struct Item {            // one queue entry (16 bytes)
 struct alignas(16) ReqDesc {   // device table entry of an admitted request
     const uint4* W;      // grid: packed weights
     const int4* idx;     // grid: packed stencil indices
-    const double* PT;    // grid: pointwise records
+    const double* PTl;   // grid: tile-transposed pointwise values
     const double* Wl;    // grid: tile-transposed weights (node-per-lane split)
     const int* idxl;     // grid: tile-transposed stencil indices
     int n;               // nodes
@@ -136,14 +136,16 @@ __device__ __forceinline__ void serve_epilogue(const ReqDesc& r, int stage, long
                                const double* __restrict__ Kin, double* __restrict__ Kout, double* __restrict__ Dm) {
     double q[4], F[4];
     load_row_cg(Kin + 4 * i, q);
-    pointwise_rhs(acc, q, r.PT + i * kPointStride, r.gh0, F);
+    double pt[kPointFields];
+    lane::points(r.PTl, i / kLaneTile, (int)(i % kLaneTile), pt);
+    pointwise_rhs(acc, q, pt, r.gh0, F);
     const double dt = r.dt;
     if (stage == 0) {
         double kn[4];
 #pragma unroll
         for (int x = 0; x < 4; ++x) kn[x] = Quad<double>::axpy(q[x], dt / 2.0, F[x]);
-        Quad<double>::store_row(Dm + 4 * i, F);
-        Quad<double>::store_row(Kout + 4 * i, kn);
+        lane::put_row(Dm + 4 * i, F);
+        lane::put_row(Kout + 4 * i, kn);
     } else {
         double h[4], d[4];
         load_row_cg(Hm + 4 * i, h);
@@ -156,15 +158,15 @@ __device__ __forceinline__ void serve_epilogue(const ReqDesc& r, int stage, long
                 d[x] = Quad<double>::axpy(d[x], 2.0, F[x]);
                 kn[x] = Quad<double>::axpy(h[x], c, F[x]);
             }
-            Quad<double>::store_row(Dm + 4 * i, d);
-            Quad<double>::store_row(Kout + 4 * i, kn);
+            lane::put_row(Dm + 4 * i, d);
+            lane::put_row(Kout + 4 * i, kn);
         } else {
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
                 d[x] = Quad<double>::axpy(d[x], 1.0, F[x]);
                 h[x] = Quad<double>::update_h(h[x], dt / 6.0, d[x]);
             }
-            Quad<double>::store_row(Hm + 4 * i, h);
+            lane::put_row(Hm + 4 * i, h);
         }
     }
 }
@@ -359,6 +361,7 @@ struct Grid {
     void* W = nullptr;
     int* idx = nullptr;
     void* PT = nullptr;
+    void* PTl = nullptr;
     void* Wl = nullptr;     // tile-transposed copies for the node-per-lane split
     int* idxl = nullptr;
 };
@@ -547,7 +550,7 @@ struct Server {
         ReqDesc d{};
         d.W = reinterpret_cast<const uint4*>(G.W);
         d.idx = reinterpret_cast<const int4*>(G.idx);
-        d.PT = reinterpret_cast<const double*>(G.PT);
+        d.PTl = reinterpret_cast<const double*>(G.PTl);
         d.Wl = reinterpret_cast<const double*>(G.Wl);
         d.idxl = G.idxl;
         d.n = G.n;
@@ -847,6 +850,7 @@ int swe_srv_add_grid(int n, int nnbr, double gh0, double dt, const int* idx, con
     G.W = ps.W;
     G.idx = ps.idx;
     G.PT = ps.PT;
+    G.PTl = ps.PTl;
     G.Wl = ps.Wl;
     G.idxl = ps.idxl;
     // the 16-bit offsets are not read here: a second index path in the persistent
@@ -1022,6 +1026,7 @@ int swe_srv_stop(void) {
         cudaFree(G.W);
         cudaFree(G.idx);
         cudaFree(G.PT);
+        cudaFree(G.PTl);
         cudaFree(G.Wl);
         cudaFree(G.idxl);
     }

@@ -20,6 +20,10 @@
 // gather touches 19 of 32 lines against 24 in slot order).  N=40962 FP64: 10.2 us
 // per stage with 128-bit loads, 8.7 with 256-bit loads, 8.2 with sorted slots;
 // N=10242 5.1 / 4.1 / 4.1; N=655362 134.3 / 133.2 / 133.0.
+// The pointwise values are transposed the same way: a record per node puts each field's
+// load on 32 lines, a third of the L1 sectors of a whole stage: us per stage
+// with records / transposed FP64 N=75000 13.3 / 11.8, N=163842 30.1 / 27.9, N=655362 126.5 /
+// 120.6, FP32 N=655362 65.2 / 63.0.
 // Weights and indices are streamed with L1 no-allocate loads; the
 // neighbour gathers keep L1 to themselves.  One warp per unit of 32 / LPN nodes,
 // no persistent loop: the hardware scheduler balances the tail.  MINB (4 or 5)
@@ -45,7 +49,8 @@ constexpr int kLaneTile = 32;      // nodes per transposed tile of the packed ar
 // FP64 N=40962 8.2 / 9.2 (weights 42 MB, below the line), N=60000 13.3 / 13.3, N=90000
 // 21.0 / 17.6, N=163842 36.4 / 30.3, N=655362 131.7 / 126.1; FP32 N=125000 14.8 / 14.4,
 // N=163842 18.4 / 14.9, N=655362 71.7 / 65.2.  Keeping 1/16, 1/8, 1/4, 1/2 or all of the
-// tiles: 31.3, 30.8, 30.3, 31.3 and 32.6 (FP64 N=163842).
+// tiles: 31.3, 30.8, 30.3, 31.3 and 32.6 (FP64 N=163842).  (Before the slots were placed and
+// the pointwise values transposed; N=163842 27.7, N=655362 120.6 and FP32 13.9 and 63.1 since.)
 constexpr int kLaneKeep = 16;      // tiles of every 64 kept in L2
 inline bool lane_streams(long n, size_t fsize) { return n * kSlots * 4 * (long)fsize > 60L * 1000 * 1000; }
 
@@ -53,6 +58,7 @@ template <typename T>
 struct LaneArgs {
     StageArgs<T> s;
     const T* Wl;       // [tile][slot][32 nodes][4] weights (Dx, Dy, Dz, L)
+    const T* PTl;      // [tile][kPointFields][32 nodes] pointwise values
     const int* idxl;   // [tile][slot][32 nodes] gather rows
     const short* idxs; // the same as 16-bit offsets from the node's own row (clamped to n - 1)
     int l2_prefetch;   // 1: bulk L2 prefetch of each warp's contiguous blocks at its start
@@ -97,6 +103,13 @@ __device__ __forceinline__ uint64_t l2_policy(int stream, long tile) {
     asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
     return !stream ? l2_normal() : (tile & 63) < kLaneKeep ? last : first;
 }
+// the pointwise values of node t of a tile
+template <typename T>
+__device__ __forceinline__ void points(const T* PTl, long tile, int t, T (&pt)[kPointFields]) {
+    const T* p = PTl + tile * kPointFields * kLaneTile + t;
+#pragma unroll
+    for (int f = 0; f < kPointFields; ++f) pt[f] = __ldg(p + f * kLaneTile);
+}
 // one state row (u, v, w, h): a whole 32-byte sector in one load (FP64)
 __device__ __forceinline__ void state_row(const double* p, double (&v)[4]) {
     asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
@@ -104,6 +117,17 @@ __device__ __forceinline__ void state_row(const double* p, double (&v)[4]) {
                  : "l"(p));
 }
 __device__ __forceinline__ void state_row(const float* p, float (&v)[4]) { Quad<float>::load_row(p, v); }
+// the same for rows that this kernel writes, and the store
+__device__ __forceinline__ void own_row(const double* p, double (&v)[4]) {
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+                 : "l"(p));
+}
+__device__ __forceinline__ void own_row(const float* p, float (&v)[4]) { Quad<float>::load_row_rw(p, v); }
+__device__ __forceinline__ void put_row(double* p, const double (&v)[4]) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3]) : "memory");
+}
+__device__ __forceinline__ void put_row(float* p, const float (&v)[4]) { Quad<float>::store_row(p, v); }
 }  // namespace lane
 
 // I16: read the gather rows from the 16-bit offsets (half the index bytes); every
@@ -135,7 +159,7 @@ __global__ void __launch_bounds__(kLaneThreads, MINB) stage_lane_kernel(const La
         prefetch_l2_bulk(reinterpret_cast<const unsigned char*>(la.Wl) + tb * kTileW + wt * (kTileW / LPN), kTileW / LPN);
         const void* ib = I16 ? static_cast<const void*>(la.idxs) : static_cast<const void*>(la.idxl);
         prefetch_l2_bulk(reinterpret_cast<const unsigned char*>(ib) + tb * kTileI + wt * (kTileI / LPN), kTileI / LPN);
-        prefetch_l2_bulk(a.PT + node0 * kPointStride, (uint32_t)(nvalid * kPointStride * sizeof(T)));
+        if (wt == 0) prefetch_l2_bulk(la.PTl + tb * kPointFields * kLaneTile, (uint32_t)(kPointFields * kLaneTile * sizeof(T)));
     }
     // a warp's nodes lie in one tile of the packed arrays (kNpw divides 32); nodes
     // past n in the last tile have zero weights and gather a valid row
@@ -198,21 +222,23 @@ __global__ void __launch_bounds__(kLaneThreads, MINB) stage_lane_kernel(const La
     }
     if (sub != 0 || i >= a.n) return;
     T q[4], F[4];
-    Quad<T>::load_row(a.Kin + 4L * (i + a.pid0), q);
-    pointwise_rhs(acc, q, a.PT + i * kPointStride, a.gh0, F);
+    lane::state_row(a.Kin + 4L * (i + a.pid0), q);
+    T pt[kPointFields];
+    lane::points(la.PTl, tile, t, pt);
+    pointwise_rhs(acc, q, pt, a.gh0, F);
     if (MODE == kEvalOnly) {
-        Quad<T>::store_row(a.F + 4 * i, F);
+        lane::put_row(a.F + 4 * i, F);
     } else if (MODE == kStage0) {
         // copy_fp_arr(D, F) and eval_K(H, K, F, dt/2): here K_in is H
         T kn[4];
 #pragma unroll
         for (int x = 0; x < 4; ++x) kn[x] = Quad<T>::axpy(q[x], a.c, F[x]);
-        Quad<T>::store_row(a.D + 4 * i, F);
-        Quad<T>::store_row(a.Kout + 4 * i, kn);
+        lane::put_row(a.D + 4 * i, F);
+        lane::put_row(a.Kout + 4 * i, kn);
     } else {
         T h[4], d[4];
-        Quad<T>::load_row_rw(a.H + 4 * i, h);
-        Quad<T>::load_row_rw(a.D + 4 * i, d);
+        lane::own_row(a.H + 4 * i, h);
+        lane::own_row(a.D + 4 * i, d);
         if (MODE == kStage1 || MODE == kStage2) {
             // update_D(D, F, 2) and eval_K(H, K, F, c)
             T kn[4];
@@ -221,8 +247,8 @@ __global__ void __launch_bounds__(kLaneThreads, MINB) stage_lane_kernel(const La
                 d[x] = Quad<T>::axpy(d[x], T(2), F[x]);
                 kn[x] = Quad<T>::axpy(h[x], a.c, F[x]);
             }
-            Quad<T>::store_row(a.D + 4 * i, d);
-            Quad<T>::store_row(a.Kout + 4 * i, kn);
+            lane::put_row(a.D + 4 * i, d);
+            lane::put_row(a.Kout + 4 * i, kn);
         } else {
             // update_D(D, F, 1) and update_H(H, D, dt)
 #pragma unroll
@@ -230,7 +256,7 @@ __global__ void __launch_bounds__(kLaneThreads, MINB) stage_lane_kernel(const La
                 d[x] = Quad<T>::axpy(d[x], T(1), F[x]);
                 h[x] = Quad<T>::update_h(h[x], a.dt6, d[x]);
             }
-            Quad<T>::store_row(a.H + 4 * i, h);
+            lane::put_row(a.H + 4 * i, h);
         }
     }
 }
