@@ -66,11 +66,12 @@ __host__ __device__ constexpr int ens_a_row_node(int r) {
 
 // Column of the B operand (and of the accumulator) within a 32-column chunk that holds
 // field f of chunk member m (0..7).  T = 32: thread i's columns in a 16x256b load,
-// 8 k + 2 (i % 4) + b, are fields 0..3 of members i % 4 and i % 4 + 4 (member
-// i % 4 + 4 (k & 1), field 2 (k >> 1) + b).  T = 16: member-major, 4 m + f.
+// 8 k + 2 (i % 4) + b, are fields 0..3 of members 2 (i % 4) and 2 (i % 4) + 1 (member
+// 2 (i % 4) + (k & 1), field 2 (k >> 1) + b), whose state is 32 contiguous bytes.  T = 16:
+// member-major, 4 m + f.
 template <int T>
 __host__ __device__ constexpr int ens_b_col(int m, int f) {
-    return T == 32 ? 8 * (2 * (f >> 1) + (m >> 2)) + 2 * (m & 3) + (f & 1) : 4 * m + f;
+    return T == 32 ? 8 * (2 * (f >> 1) + (m & 1)) + 2 * (m >> 1) + (f & 1) : 4 * m + f;
 }
 
 struct EnsArgs;
@@ -78,6 +79,18 @@ struct EnsArgs;
 namespace ens {
 
 __device__ __forceinline__ float4 ldg_f4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+// two float4 at p (32-byte aligned) in one access
+__device__ __forceinline__ void ldg_2f4(const float* p, float4 (&v)[2]) {
+    asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[0].z), "=f"(v[0].w), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[1].z),
+                   "=f"(v[1].w)
+                 : "l"(p));
+}
+__device__ __forceinline__ void st_2f4(float* p, const float4 (&v)[2]) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0].x), "f"(v[0].y), "f"(v[0].z),
+                 "f"(v[0].w), "f"(v[1].x), "f"(v[1].y), "f"(v[1].z), "f"(v[1].w)
+                 : "memory");
+}
 __device__ __forceinline__ float2 ldg_f2(const float* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
 
 // hi = bf16(a, b) (round to nearest even), lo = bf16 of the remainders; packed pairs, a in the low half.
@@ -266,10 +279,10 @@ struct HalfOperands {
         int p, kh;
         __device__ explicit Thread(int ct) : p(ct % (kN / 2)), kh(ct / (kN / 2)) {}
         // member-field (state column) of B column 2p: within its 32-column chunk,
-        // 2p = 8 k + 2 i holds member i + 4 (k & 1), fields 2 (k >> 1) and + 1
+        // 2p = 8 k + 2 i holds member 2 i + (k & 1), fields 2 (k >> 1) and + 1
         __device__ int col() const {
             const int k = (p >> 2) & 3, i = p & 3;
-            return 32 * (p >> 4) + 4 * (i + 4 * (k & 1)) + 2 * (k >> 1);
+            return 32 * (p >> 4) + 4 * (2 * i + (k & 1)) + 2 * (k >> 1);
         }
     };
     struct Fetch {

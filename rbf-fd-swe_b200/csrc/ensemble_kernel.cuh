@@ -422,28 +422,46 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
             if constexpr (kScaled) tc::bulk_g2s(tb + C::kTbAi, a.AI + (long)tile * T, nn * 16, &tile_bar[b]);
         };
         // this thread's pair pi of a chunk: tile node pair_node(pi) and chunk member
-        // pair_member(pi).  32-node tiles: node qt 8 + lane / 4, members lane % 4 and
-        // lane % 4 + 4 (the columns tmem_ld16x256 gives the thread, ens_b_col);
+        // pair_member(pi).  32-node tiles: node qt 8 + lane / 4, members 2 (lane % 4) and
+        // the next (the columns tmem_ld16x256 gives the thread, ens_b_col);
         // 16-node tiles: node qt 4 + (p >> 3), member p & 7, with p = lane + 32 pi.
         auto pair_node = [&](int pi) { return T == 32 ? qt * 8 + (lane >> 2) : qt * (T / 4) + ((lane + 32 * pi) >> 3); };
-        auto pair_member = [&](int pi) { return T == 32 ? (lane & 3) + 4 * pi : (lane + 32 * pi) & 7; };
+        auto pair_member = [&](int pi) { return T == 32 ? 2 * (lane & 3) + pi : (lane + 32 * pi) & 7; };
         // streamed per-(node, member) operands of one chunk for this thread's pairs
         auto fetch = [&](int u, int ch, ens::EpiSet& o) {
             const int tile = u / halves;
             const int col0 = (u % halves) * C::kN;
-#pragma unroll
-            for (int pi = 0; pi < C::kPairs; ++pi) {
-                const long node = (long)tile * T + pair_node(pi);
-                if (node >= a.n) continue;
-                const int mfb = col0 + ch * 32 + 4 * pair_member(pi);
-                const long e4 = node * a.mf + mfb;
-                const long eh = node * members + (mfb >> 2);
-                o.own[pi] = ens::ldg_f4(a.Kin + e4);
-                if (MODE != kEvalOnly) o.hh[pi] = __ldg(a.Hh + eh);
+            if constexpr (T == 32) {                 // both pairs' operands lie together
+                const long node = (long)tile * T + pair_node(0);
+                if (node >= a.n) return;
+                const int mfb = col0 + ch * 32 + 4 * pair_member(0);
+                const long e4 = node * a.mf + mfb, eh = node * members + (mfb >> 2);
+                auto two = [](const double* p, double (&v)[2]) {
+                    const double2 d = __ldg(reinterpret_cast<const double2*>(p));
+                    v[0] = d.x; v[1] = d.y;
+                };
+                ens::ldg_2f4(a.Kin + e4, o.own);
+                if (MODE != kEvalOnly) two(a.Hh + eh, o.hh);
                 if (kHD) {
-                    o.h32[pi] = ens::ldg_f4(a.H32 + e4);
-                    o.d32[pi] = ens::ldg_f4(a.D32 + e4);
-                    o.dh[pi] = __ldg(a.Dh + eh);
+                    ens::ldg_2f4(a.H32 + e4, o.h32);
+                    ens::ldg_2f4(a.D32 + e4, o.d32);
+                    two(a.Dh + eh, o.dh);
+                }
+            } else {
+#pragma unroll
+                for (int pi = 0; pi < C::kPairs; ++pi) {
+                    const long node = (long)tile * T + pair_node(pi);
+                    if (node >= a.n) continue;
+                    const int mfb = col0 + ch * 32 + 4 * pair_member(pi);
+                    const long e4 = node * a.mf + mfb;
+                    const long eh = node * members + (mfb >> 2);
+                    o.own[pi] = ens::ldg_f4(a.Kin + e4);
+                    if (MODE != kEvalOnly) o.hh[pi] = __ldg(a.Hh + eh);
+                    if (kHD) {
+                        o.h32[pi] = ens::ldg_f4(a.H32 + e4);
+                        o.d32[pi] = ens::ldg_f4(a.D32 + e4);
+                        o.dh[pi] = __ldg(a.Dh + eh);
+                    }
                 }
             }
         };
@@ -487,6 +505,9 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
                 fetch(u, ch, o);
                 __syncwarp();
             }
+            // a pair's results: the state it writes (K, H or F), D32 and the FP64 h or D
+            float4 r4[2], rd[2];
+            double rh[2];
 #pragma unroll
             for (int pi = 0; pi < C::kPairs; ++pi) {
                 const int t = pair_node(pi);
@@ -546,43 +567,51 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
                 pointwise_rhs<float>(S, q, pt, a.gh0, F);
                 const long e4 = node * a.mf + mfb;
                 const long eh = node * members + member;
+                const double fh = (double)F[3];
                 if (MODE == kEvalOnly) {
-                    *reinterpret_cast<float4*>(a.F + e4) = make_float4(F[0], F[1], F[2], F[3]);
+                    r4[pi] = make_float4(F[0], F[1], F[2], F[3]);
                 } else if (MODE == kStage0) {
                     // K = H + c F (q is the base state here); D = F
-                    const double fh = (double)F[3];
-                    *reinterpret_cast<float4*>(a.D32 + e4) = make_float4(F[0], F[1], F[2], 0.f);
-                    a.Dh[eh] = fh;
-                    *reinterpret_cast<float4*>(a.Kout + e4) =
-                        make_float4(__fadd_rn(q[0], __fmul_rn(c32, F[0])), __fadd_rn(q[1], __fmul_rn(c32, F[1])),
-                                    __fadd_rn(q[2], __fmul_rn(c32, F[2])), __double2float_rn(o.hh[pi] + a.c * fh));
+                    rd[pi] = make_float4(F[0], F[1], F[2], 0.f);
+                    rh[pi] = fh;
+                    r4[pi] = make_float4(__fadd_rn(q[0], __fmul_rn(c32, F[0])), __fadd_rn(q[1], __fmul_rn(c32, F[1])),
+                                         __fadd_rn(q[2], __fmul_rn(c32, F[2])), __double2float_rn(o.hh[pi] + a.c * fh));
                 } else if (MODE == kStage1 || MODE == kStage2) {
-                    const double fh = (double)F[3];
                     const float4 h4 = o.h32[pi], d4 = o.d32[pi];
-                    *reinterpret_cast<float4*>(a.D32 + e4) =
-                        make_float4(__fadd_rn(d4.x, __fmul_rn(2.f, F[0])), __fadd_rn(d4.y, __fmul_rn(2.f, F[1])),
-                                    __fadd_rn(d4.z, __fmul_rn(2.f, F[2])), 0.f);
-                    a.Dh[eh] = o.dh[pi] + 2.0 * fh;
-                    *reinterpret_cast<float4*>(a.Kout + e4) =
-                        make_float4(__fadd_rn(h4.x, __fmul_rn(c32, F[0])), __fadd_rn(h4.y, __fmul_rn(c32, F[1])),
-                                    __fadd_rn(h4.z, __fmul_rn(c32, F[2])), __double2float_rn(o.hh[pi] + a.c * fh));
+                    rd[pi] = make_float4(__fadd_rn(d4.x, __fmul_rn(2.f, F[0])), __fadd_rn(d4.y, __fmul_rn(2.f, F[1])),
+                                         __fadd_rn(d4.z, __fmul_rn(2.f, F[2])), 0.f);
+                    rh[pi] = o.dh[pi] + 2.0 * fh;
+                    r4[pi] = make_float4(__fadd_rn(h4.x, __fmul_rn(c32, F[0])), __fadd_rn(h4.y, __fmul_rn(c32, F[1])),
+                                         __fadd_rn(h4.z, __fmul_rn(c32, F[2])), __double2float_rn(o.hh[pi] + a.c * fh));
                 } else {
                     const float4 h4 = o.h32[pi], d4 = o.d32[pi];
                     const float du = __fadd_rn(d4.x, F[0]), dv = __fadd_rn(d4.y, F[1]), dw = __fadd_rn(d4.z, F[2]);
-                    const double dh = o.dh[pi] + (double)F[3];
+                    const double dh = o.dh[pi] + fh;
                     const double h = o.hh[pi] + a.dt6 * dh;
-                    a.Hh[eh] = h;
+                    rh[pi] = h;
                     const float4 hn = make_float4(__double2float_rn((double)h4.x + a.dt6 * (double)du),
                                                   __double2float_rn((double)h4.y + a.dt6 * (double)dv),
                                                   __double2float_rn((double)h4.z + a.dt6 * (double)dw),
                                                   __double2float_rn(h));
-                    *reinterpret_cast<float4*>(a.H32 + e4) = hn;
+                    r4[pi] = hn;
                     if constexpr (PREC == kFp16x3) {
                         hmax[0] = max(hmax[0], __float_as_uint(fabsf(hn.x)));
                         hmax[1] = max(hmax[1], __float_as_uint(fabsf(hn.y)));
                         hmax[2] = max(hmax[2], __float_as_uint(fabsf(hn.z)));
                         hmax[3] = max(hmax[3], __float_as_uint(fabsf(hn.w)));
                     }
+                }
+                float* out = MODE == kEvalOnly ? a.F : MODE == kStage3 ? a.H32 : a.Kout;
+                double* outh = MODE == kStage3 ? a.Hh : a.Dh;
+                constexpr bool kD = MODE == kStage0 || MODE == kStage1 || MODE == kStage2;
+                if constexpr (T != 32) {
+                    *reinterpret_cast<float4*>(out + e4) = r4[pi];
+                    if (kD) *reinterpret_cast<float4*>(a.D32 + e4) = rd[pi];
+                    if (MODE != kEvalOnly) outh[eh] = rh[pi];
+                } else if (pi == 1) {                // both pairs at once: e4 and eh are the second's
+                    ens::st_2f4(out + e4 - 4, r4);
+                    if (kD) ens::st_2f4(a.D32 + e4 - 4, rd);
+                    if (MODE != kEvalOnly) *reinterpret_cast<double2*>(outh + eh - 1) = make_double2(rh[0], rh[1]);
                 }
             }
             if constexpr (T != 32) __syncwarp();   // the exchange rows are rewritten by the next chunk
