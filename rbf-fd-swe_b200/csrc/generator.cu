@@ -290,7 +290,8 @@ __device__ __forceinline__ double ipow(double x, int e) {
 // 2 i + h: 3 x 25 values, so the two half-warps share every row and the trailing columns
 // of an elimination step stay spread over all lanes.  Rows and columns 0..31 are the RBF
 // block, 32..46 the polynomials, columns 47..49 the right-hand sides; places k..31 of a
-// stencil of k < 32 nodes hold zeros and their steps are skipped.
+// stencil of k < 32 nodes hold zeros and their steps are skipped (from column 15 on; before,
+// they hold a row of the identity, which costs the wide stencils no branch).
 //
 // A step picks the largest |entry| of its column among the rows not yet used (its leading
 // bits and row number in one 32-bit maximum over the warp: the largest to within 2^-14,
@@ -382,7 +383,7 @@ weights_kernel(const double* __restrict__ X, const int* __restrict__ idx, int n,
                     const double t = a * a + b * b;
                     v = (t * t) * (t * t) * sqrt(t);              // r^9
                 }
-                m[s][i] = rv && c < k ? v : 0.0;
+                m[s][i] = rv && c < k ? v : c == r && r < kNPoly ? 1.0 : 0.0;
             }
 #pragma unroll
             for (int i = 16; i < 23; ++i) m[s][i] = rv ? w.poly[r * kPolyLd + 2 * (i - 16) + h] : 0.0;

@@ -114,3 +114,18 @@ def test_weights_of_coincident_nodes_are_refused():
     X[idx[100, 5]] = X[idx[100, 4]]
     with pytest.raises(capi.SweError, match="singular"):
         gen.rbffd_weights_gpu(X, idx)
+
+
+@pytest.mark.parametrize("k", [3, 5, 12, 14])
+def test_stencils_below_the_polynomial_count_are_accepted(k):
+    """Fewer nodes than the 15 polynomials: the systems have no unique solution and their
+    weights are rounding, but the call is accepted (k = 1, a stencil without extent, is not)."""
+    t = np.arange(500) + 0.5
+    z = 1.0 - t / 250.0
+    r = np.sqrt(1.0 - z * z)
+    a = np.pi * (1 + 5 ** 0.5) * t
+    X = np.stack([r * np.cos(a), r * np.sin(a), z], 1)
+    for D in gen.rbffd_weights_gpu(X, gen.stencils_gpu(X, k)):
+        assert np.isfinite(D).all()
+    with pytest.raises(capi.SweError, match="singular"):
+        gen.rbffd_weights_gpu(X, gen.stencils_gpu(X, 1))
