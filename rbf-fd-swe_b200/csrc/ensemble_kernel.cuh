@@ -29,8 +29,9 @@
 // state K are FP32.
 //
 // Persistent, warp-specialised CTA (one per SM; it owns all of tensor memory):
-//   * converter warps (MPC/8): for each 16-row chunk of K they gather the rows
-//     as async copies into a staging buffer issued two chunks ahead, three
+//   * converter warps (MPC/8 in a group; one group for 64 members, two on alternate
+//     chunks for 32): for each 16-row chunk of K they gather the rows
+//     as async copies into a staging buffer issued two chunks of the group ahead, three
 //     buffers deep, so that no register waits on a gather (16 bytes a row for
 //     3xTF32, 8 for the 16-bit splits), and centre and split them into the B
 //     operand;
@@ -52,6 +53,18 @@
 //     thread and pair, while the tensor cores already fill the other accumulator.
 // Every mbarrier wait is bounded; a timeout sets an error word and a shared
 // abort flag that makes every role leave its loop.
+//
+// What bounds it: the state, accumulator and pointwise rows of a stage are 20 (m32 of 40,962
+// nodes) to 139 us (m64 of 163,842) of DRAM time, the tensor cores need less; the rest is
+// the converters' chain (wait, gather, split, store) and the epilogue's loads.  Measured for
+// one stage, 3xTF32 / FP16 / BF16, us:
+//   N = 163,842, 64 members: 334 / 312 / 312, with overlapped launches and odd stages from
+//   the last tile (the rows the stage before wrote last are still in L2) 328 / 306 / 308,
+//   with two adjacent members a thread in 256-bit accesses 317 / 295 / 289;
+//   N = 40,962, 32 members: 72.2 / 70.2 / 69.5, 68.9 / 67 / 66, 67.8 / 64.7 / 63.7, and with
+//   two converter groups 56.5 / 51.0 / 49.8.
+// 64 members a CTA keep one group: two would leave a thread 72 registers, and its eight
+// warps already put two on each scheduler.
 #pragma once
 
 #include "ens_operands.cuh"
@@ -72,10 +85,14 @@ struct EnsCfg {
     static constexpr int kN = 4 * MPC;                     // MMA N: member-fields per CTA
     static constexpr int kConvWarps = MPC / 8;             // 4 * MPC converter threads
     static constexpr int kConvThreads = 32 * kConvWarps;
-    static constexpr int kMmaWarp = kConvWarps;
-    static constexpr int kEpiWarp0 = kConvWarps + 1;
+    // with 32 members a group is four warps, one per scheduler: two groups take alternate
+    // chunks, or each chunk's chain of waits, copies and conversions runs by itself (one
+    // group 64.7 us a stage at N = 40,962 with split FP16, two 51.0)
+    static constexpr int kGroups = MPC == 32 ? 2 : 1;
+    static constexpr int kMmaWarp = kGroups * kConvWarps;
+    static constexpr int kEpiWarp0 = kMmaWarp + 1;
     static constexpr int kProdWarp = kEpiWarp0 + kEnsEpiWarps;   // A operand producer
-    static constexpr int kThreads = 32 * (kConvWarps + 2 + kEnsEpiWarps);
+    static constexpr int kThreads = 32 * (kMmaWarp + 2 + kEnsEpiWarps);
     static constexpr int kStages = Op::kStages;            // ring slots
     static constexpr int kStageBytes = Op::kStageBytes;
     static constexpr int kXchStride = 36;                  // floats per (op, node) row; 9 x 16 B
@@ -88,7 +105,7 @@ struct EnsCfg {
     static constexpr int kTbAi = kTbCen + kN * 4;          // FP16 operands: the tile's A-row inverse scales
     static constexpr int kTileBuf = (kTbAi + T * 16 + 127) / 128 * 128;
     static constexpr int kStgOff = kStages * kStageBytes + kEnsEpiWarps * kXchWarpFloats * 4 + 2 * kTileBuf;
-    static constexpr int kSmem = kStgOff + Op::kStgDepth * Op::kStgBytes;
+    static constexpr int kSmem = kStgOff + kGroups * Op::kStgDepth * Op::kStgBytes;
     static constexpr int kTmemCols = (2 * kN <= 256) ? 256 : 512;
     static_assert(kConvThreads == Op::kConvThreads, "converter thread count");
     static_assert(kSmem + 1024 <= 227 * 1024, "dynamic shared memory beside the barriers fits 227 KB");
@@ -253,7 +270,7 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
     tc::fence_after_sync();
     const uint32_t tmem = tmem_s;
 
-    if (warp < C::kConvWarps) {
+    if (warp < C::kMmaWarp) {
         // =============================== converters ===============================
         // FP16 operands: this thread's two fields (f0, f0 + 1) and their scales
         float2 sc = make_float2(1.f, 1.f);
@@ -268,30 +285,37 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
                 if constexpr (MODE == kStage0) a.bmax_pub[threadIdx.x] = a.bmax[threadIdx.x];
                 if constexpr (MODE == kStage2) a.bmax_next[threadIdx.x] = 0u;
             }
-            const int f0 = typename Op::Thread(threadIdx.x).col() & 3;
+            const int f0 = typename Op::Thread(threadIdx.x % C::kConvThreads).col() & 3;
             sc = make_float2(ens::fp16_field_scale(a.bmax, f0, false), ens::fp16_field_scale(a.bmax, f0 + 1, false));
         }
-        // staged gathers: chunk g + 2's rows are in flight (cp.async) while chunk g is
-        // built from its staging buffer
-        const typename Op::Thread th(threadIdx.x);
-        const int ct = threadIdx.x;
-        unsigned char* stg0 = smem + C::kStgOff;
-        // chunk g's gathers are issued two steps ahead as async copies into staging
-        // buffer g % 3; the centre row of a new unit is loaded into a register then too
+        // staged gathers: the rows of this group's chunk after next are in flight (cp.async)
+        // while a chunk is built from its staging buffer
+        const int ct = threadIdx.x % C::kConvThreads, group = threadIdx.x / C::kConvThreads;
+        const typename Op::Thread th(ct);
+        unsigned char* stg0 = smem + C::kStgOff + group * (Op::kStgDepth * Op::kStgBytes);
+        auto next = [&](ens::Cursor p) {
+#pragma unroll
+            for (int k = 0; k < C::kGroups; ++k) p = ens::next_cursor<MODE>(p, a, halves);
+            return p;
+        };
+        // a chunk's gathers are issued two of the group's steps ahead as async copies into
+        // one of three staging buffers; the centre row of a new unit is loaded into a
+        // register then too
         ens::Cursor cur = ens::first_cursor<MODE>(a, halves);
-        ens::Cursor c1 = ens::next_cursor<MODE>(cur, a, halves);
-        ens::Cursor c2 = ens::next_cursor<MODE>(c1, a, halves);
-        typename Op::Fetch f2, f3;     // indices of chunks g + 2 and g + 3
+        if (group == 1) cur = ens::next_cursor<MODE>(cur, a, halves);
+        ens::Cursor c1 = next(cur);
+        ens::Cursor c2 = next(c1);
+        typename Op::Fetch f2, f3;     // indices of the group's second and third chunk from here
         using Cen = typename Op::Cen;
-        Cen cen0{}, cen1{}, cen2{};    // centres of chunks g, g+1, g+2
+        Cen cen0{}, cen1{}, cen2{};    // centres of its present and next two chunks
         // returns the centre state of chunk p's unit (a new unit loads it; else prev)
-        auto issue = [&](const ens::Cursor& p, const typename Op::Fetch& f, int slot, Cen prev) {
+        auto issue = [&](const ens::Cursor& p, const typename Op::Fetch& f, int slot, bool fresh, Cen prev) {
             Cen c = prev;
             if (p.valid) {
                 const int unit = ens::unit_at<MODE>(a, p.u), tile = unit / halves;
                 const long col = (long)(unit % halves) * C::kN + th.col();
                 Op::stage_issue(stg0 + slot * Op::kStgBytes, ct, a.Kin, a.mf, col, f);
-                if (p.gc == p.gc0) c = Op::load_cen(a.Kin + (long)__ldg(a.centre + tile) * a.mf + col);
+                if (fresh) c = Op::load_cen(a.Kin + (long)__ldg(a.centre + tile) * a.mf + col);
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
             return c;
@@ -301,25 +325,26 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
             Op::fetch_idx(a.rows, cur.gc, th, f0);
             if (c1.valid) Op::fetch_idx(a.rows, c1.gc, th, f1);
             if (c2.valid) Op::fetch_idx(a.rows, c2.gc, th, f2);
-            cen0 = issue(cur, f0, 0, cen0);
-            cen1 = issue(c1, f1, 1, cen0);
+            cen0 = issue(cur, f0, 0, true, cen0);
+            cen1 = issue(c1, f1, 1, c1.ti != cur.ti, cen0);
         }
-        int g = 0;
+        int g = group, k = 0;          // chunk of the CTA, chunk of the group
         while (cur.valid) {
-            // chunk g + 2's gathers, chunk g + 3's indices
-            cen2 = issue(c2, f2, (g + 2) % 3, cen1);
-            const ens::Cursor c3 = ens::next_cursor<MODE>(c2, a, halves);
+            // the gathers of the group's chunk after next, the indices of the one after that
+            cen2 = issue(c2, f2, (k + 2) % 3, c2.ti != c1.ti, cen1);
+            const ens::Cursor c3 = next(c2);
             if (c3.valid) Op::fetch_idx(a.rows, c3.gc, th, f3);
             asm volatile("cp.async.wait_group 2;" ::: "memory");
             const int s = g % C::kStages;
             if (!ens::wait(&empty_bar[s], ((g / C::kStages) & 1) ^ 1, abort_v, a.err, 3)) break;
             typename Op::Set o;
-            Op::stage_read(stg0 + (g % 3) * Op::kStgBytes, ct, cen0, o);
+            Op::stage_read(stg0 + (k % 3) * Op::kStgBytes, ct, cen0, o);
             Op::build(smem + s * C::kStageBytes, th, o, sc, cur.gc + 1 == cur.gc_end);
             tc::fence_async_smem();
             __syncwarp();
             if (lane == 0) ens::mbar_arrive(&full_bar[s]);
-            ++g;
+            g += C::kGroups;
+            ++k;
             cur = c1;
             c1 = c2;
             c2 = c3;
