@@ -225,7 +225,12 @@ extern "C" int swe_dev_rcm_mapping(int n, int nnbr, const int* idx, int* mapping
     }
     if (mem) cudaFree(mem);
     if (st) cudaStreamDestroy(st);
-    if (e != cudaSuccess) {
+    // a bad index is reported before any CUDA error: where the device did not get to check
+    // (no device, no memory), the host does
+    if (e != cudaSuccess)
+        for (size_t t = 0; t < count && res.bad == ~0ull; ++t)
+            if (idx[t] < 0 || idx[t] >= n) res.bad = t;
+    if (e != cudaSuccess && res.bad == ~0ull) {
         set_error("swe_dev_rcm_mapping: %s", cudaGetErrorString(e));
         return SWE_ERR_CUDA;
     }
