@@ -361,8 +361,8 @@ int swe_srv_test_withhold(int request, int stage_index);
  * and must be serialised by the caller.  Kernels go to `stream` (a
  * cudaStream_t, NULL for the default stream); the call returns once they are
  * enqueued.  Grids of a few thousand nodes or more whose static data fits in the
- * SMs' shared memory step in one kernel that holds all SMs.  Every idx entry must lie in 0..n-1.  The kernels check each one
- * as they gather: an entry outside that range is never dereferenced (the node's
+ * SMs' shared memory step in one kernel that holds all SMs.  Every idx entry
+ * must lie in 0..n-1.  The kernels check each one as they gather: an entry outside that range is never dereferenced (the node's
  * own row is read in its place, so that call's results are wrong) and the
  * first one is recorded.  A call with nsteps = 0 steps nothing: it waits for
  * `stream` and returns SWE_ERR_INDEX, naming the recorded (node, slot, value)

@@ -8,9 +8,9 @@
 // device once and rearranged there by three kernels into every layout the stage
 // kernels read:
 //   * W / idx:   the 8-lanes-per-node layout (stage_kernel.cuh, stage_tma.cuh),
-//   * Wl / idxl: the tile-transposed node-per-lane layout (stage_lane.cuh), each
-//     node's slots placed so that neighbouring lanes gather the same lines, and
-//     idxs, the same indices as 16-bit offsets from each node's own row,
+//   * Wl / idxl: the tile-transposed node-per-lane layout (stage_lane.cuh), the
+//     slots of small patches placed so that neighbouring lanes gather the same
+//     lines, and idxs, the same indices as 16-bit offsets from each node's own row,
 //   * PT:        the pointwise records [node][kPointStride], and PTl, the same
 //     values tile-transposed for the node-per-lane kernels.
 // Slots j >= nnbr get zero weights and gather the node's own row; nodes past n in
@@ -79,16 +79,26 @@ __global__ void pack_stencils_kernel(const T* __restrict__ Dx, const T* __restri
 
 // The node-per-lane layout: one warp per group of 128 / sizeof(row) consecutive nodes (4 in
 // FP64, 8 in FP32), whose lanes gather one slot's rows in one pass of the L1 data pipe.  A
-// pass costs a cycle per distinct 128-byte line, so the group's neighbours are placed to
-// share lines: the first node's in ascending order of rows, every further node's into slots
+// pass costs a cycle per distinct 128-byte line, so with `place` the group's neighbours are
+// placed to share lines: the first node's alternately from both ends of the ascending order
+// of rows (neighbours on opposite sides cancel at once), every further node's into slots
 // whose line another node of the group already reads, the rest into the slots left, in
-// ascending order.  Lines per 32 gathered rows, sorted slots / these (N=40962, reverse
+// the same order.  Lines per 32 gathered rows, sorted slots / these (N=40962, reverse
 // Cuthill-McKee order): FP64 19.0 / 15.1, FP32 10.9 / 9.4; on a spiral of 30000 nodes FP64
 // 24.7 / 18.5, FP32 17.9 / 12.9.
+//
+// `place` holds up to kPlacedNodes: there two or more lanes share a node, and their sums are
+// as exact as those of the caller's order or more so (FP32 right-hand side of N=40962 against
+// 64 bits: 4.0e-5 in the caller's order, 1.9e-5 placed).  Above, one lane sums a node's 32
+// terms, and the caller's order, nearest first, is the more exact one (N=163842: 1.8e-5
+// against 3.1e-5 placed, 3.6e-5 sorted), at little cost: a stage of N=40962 FP64 takes 8.0 us
+// in the caller's order and 7.2 placed, of 75,000 12.0 and 11.8, of 163,842 28.2 and 28.0,
+// FP32 14.9 and 14.9, of 100,000 11.3 and 10.3.
+constexpr int kPlacedNodes = 148 * 5 * (kLaneThreads / 2);   // two lanes a node at 5 CTAs per SM fill the GPU once
 template <typename T>
 __global__ void pack_lanes_kernel(const T* __restrict__ Dx, const T* __restrict__ Dy, const T* __restrict__ Dz,
                                   const T* __restrict__ L, const int* __restrict__ idx_raw, CallerLayout cl, int n,
-                                  long npad, int nnbr, int rows, int pid0, T* __restrict__ Wl, int* __restrict__ idxl,
+                                  long npad, int nnbr, int rows, int pid0, bool place, T* __restrict__ Wl, int* __restrict__ idxl,
                                   short* __restrict__ idxs, int* __restrict__ wide) {
     constexpr int kGroup = 32 / (int)sizeof(T);      // nodes whose rows fill a pass
     constexpr int kRowsPerLine = 32 / (int)sizeof(T);
@@ -100,7 +110,8 @@ __global__ void pack_lanes_kernel(const T* __restrict__ Dx, const T* __restrict_
     int have[kGroup];                                // lines this lane's slot reads so far
     for (int t = 0; t < kGroup; ++t) {
         const long i = i0 + t;
-        // the node's rows in ascending order (ties in slot order), one a lane
+        // the node's rows, one a lane: alternately from both ends of their ascending order
+        // (ties in slot order), or as given
         int p = i < n ? (int)i + pid0 : pid0, pos = lane, src = lane;
         if (i < n) {
             if (lane < nnbr) {
@@ -108,12 +119,13 @@ __global__ void pack_lanes_kernel(const T* __restrict__ Dx, const T* __restrict_
                 if (q >= 0 && q < rows) p = q;
             }
             int rank = lane;
-            if (lane < nnbr) {
+            if (place && lane < nnbr) {
                 rank = 0;
                 for (int o = 0; o < nnbr; ++o) {
                     const int q = __shfl_sync(nnbr < 32 ? (1u << nnbr) - 1 : 0xffffffffu, p, o);
                     rank += q < p || (q == p && o < lane);
                 }
+                rank = 2 * rank < nnbr ? 2 * rank : 2 * (nnbr - 1 - rank) + 1;
             }
             __syncwarp();
             s_row[warp][rank] = p;
@@ -122,7 +134,7 @@ __global__ void pack_lanes_kernel(const T* __restrict__ Dx, const T* __restrict_
             p = s_row[warp][lane];
             src = s_src[warp][lane];
             const int line = p / kRowsPerLine;
-            if (t > 0) {
+            if (place && t > 0) {
                 const unsigned used = nnbr < 32 ? (1u << nnbr) - 1 : 0xffffffffu;
                 unsigned open = used;                // slots not taken
                 pos = lane < nnbr ? -1 : lane;
@@ -271,7 +283,7 @@ int pack_static_device(const CallerLayout& cl, int n, int rows, int pid0, int nn
     pack_stencils_kernel<T><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(tDx, tDy, tDz, tL, tidx, cl, n, nnbr,
                                                                               rows, pid0, out.W, out.idx, bad);
     pack_lanes_kernel<T><<<(unsigned)((groups + 7) / 8), 256, 0, st>>>(tDx, tDy, tDz, tL, tidx, cl, n, npad, nnbr, rows,
-                                                                      pid0, out.Wl, out.idxl, out.idxs, wide);
+                                                                      pid0, n <= kPlacedNodes, out.Wl, out.idxl, out.idxs, wide);
     pack_points_kernel<T><<<(unsigned)((npad + 255) / 256), 256, 0, st>>>(tx, ty, tz, tf, tghm, tpu, tpv, tpw, tgg, cl,
                                                                          n, npad, out.PT, out.PTl);
     count_launch(3);

@@ -125,9 +125,10 @@ __device__ __forceinline__ void load_row_l1(const double* p, double (&v)[4]) {
 // work item (or pad the last tile): they are computed on valid rows and not stored.
 // Bound by the latency of the gathers in flight (128 registers a thread).  A saturated mix of
 // 32 requests over four grids: 5.96e9 node-stages/s with a row per slot read in the loop, both
-// members finished by one lane and L2-only gathers, 6.60e9 now; work items of 1024 nodes
-// instead of 2048: 5.47e9, claiming more items while one waits for its neighbours: 6.65e9,
-// but a burst of 12 small requests 33-37 ms instead of 28.
+// members finished by one lane and L2-only gathers, 6.60e9 without, 6.90e9 with the pointwise
+// values transposed as well; work items of 1024 nodes instead of 2048 (before that): 5.47e9,
+// claiming more items while one waits for its neighbours: 6.65e9, but a burst of 12 small
+// requests 33-37 ms instead of 28.
 constexpr int kSrvLpn = 2, kSrvNpw = 32 / kSrvLpn;
 constexpr int kSrvMB = 2;   // members per work item: each weight and index is loaded once for them
 static_assert(kSrvMB == 2, "serve_kernel dispatches blocks of one or two members");

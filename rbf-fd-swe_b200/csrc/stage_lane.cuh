@@ -3,8 +3,8 @@
 // Same stage semantics as stage_kernel.cuh (eval_RHS_swe plus the RK4 stage
 // combine, swe_code/main/rk4_rbffd_swe.c:30-186 and :285-353), with a work split
 // that needs little or no cross-lane reduction: each of a node's LPN lanes (1, 2
-// or 4) sums the slots j = sub, sub + LPN, ... of the node serially, in ascending
-// order of the neighbours' rows, and the LPN partial sums meet in a butterfly of
+// or 4) sums the slots j = sub, sub + LPN, ... of the node serially, in the order
+// of the packed arrays, and the LPN partial sums meet in a butterfly of
 // log2(LPN) shuffle steps.  Lane sub 0 of every node then
 // runs the pointwise part and the stage combine, so up to all 32 lanes of a warp
 // are busy in the epilogue.
@@ -13,13 +13,12 @@
 // (pack_stencils_kernel in pack.cuh): per 32-node tile, slot-major, node-minor,
 // so one slot's weights of a warp's nodes are one contiguous 1024-byte (FP64) or
 // 512-byte (FP32) row and one slot's indices a contiguous 64- or 128-byte row.
-// Weights and FP64 state rows move as whole 32-byte sectors (256-bit loads), and
-// a node's slots are sorted by row: the L1 data pipe is what the kernel spends
-// most on when the data is in L2, and with sorted slots the lanes of a warp gather
-// neighbouring rows (N=40962, reverse Cuthill-McKee order: a 4-lane pass of a FP64
-// gather touches 19 of 32 lines against 24 in slot order).  N=40962 FP64: 10.2 us
-// per stage with 128-bit loads, 8.7 with 256-bit loads, 8.2 with sorted slots;
-// N=10242 5.1 / 4.1 / 4.1; N=655362 134.3 / 133.2 / 133.0.
+// Weights and FP64 state rows move as whole 32-byte sectors (256-bit loads): the L1
+// data pipe is what the kernel spends most on when the data is in L2.  On small
+// patches the slots are placed so that the lanes of a warp gather the same lines
+// (pack_lanes_kernel has the rule).  N=40962 FP64: 10.2 us per stage with 128-bit
+// loads, 8.7 with 256-bit loads, 7.7 with placed slots and the pointwise values
+// transposed; N=10242 5.1 / 4.1 with 128- / 256-bit loads, N=655362 134.3 / 133.2.
 // The pointwise values are transposed the same way: a record per node puts each field's
 // load on 32 lines, a third of the L1 sectors of a whole stage: us per stage
 // with records / transposed FP64 N=75000 13.3 / 11.8, N=163842 30.1 / 27.9, N=655362 126.5 /
@@ -50,7 +49,7 @@ constexpr int kLaneTile = 32;      // nodes per transposed tile of the packed ar
 // 21.0 / 17.6, N=163842 36.4 / 30.3, N=655362 131.7 / 126.1; FP32 N=125000 14.8 / 14.4,
 // N=163842 18.4 / 14.9, N=655362 71.7 / 65.2.  Keeping 1/16, 1/8, 1/4, 1/2 or all of the
 // tiles: 31.3, 30.8, 30.3, 31.3 and 32.6 (FP64 N=163842).  (Before the slots were placed and
-// the pointwise values transposed; N=163842 27.7, N=655362 120.6 and FP32 13.9 and 63.1 since.)
+// the pointwise values transposed; N=163842 28.2, N=655362 120.6 and FP32 14.9 and 63.6 since.)
 constexpr int kLaneKeep = 16;      // tiles of every 64 kept in L2
 inline bool lane_streams(long n, size_t fsize) { return n * kSlots * 4 * (long)fsize > 60L * 1000 * 1000; }
 

@@ -35,3 +35,22 @@ def test_steps_equal_substeps_bitwise_and_match_oracle(prec, n, nnbr):
         p.finalize()
     want = oracle.Port(m, prec).run(H0, 30)
     assert scaled_err(got[30], want).max() <= (1e-12 if prec == "fp64" else 1e-4)
+
+
+@pytest.mark.parametrize("n", [47361, 60001])
+def test_fp32_rhs_of_one_lane_per_node_is_as_exact_as_the_restatement(n):
+    """Above 47,360 nodes one lane sums a node's slots: in the caller's order, as the FP32
+    restatement does, with fewer roundings (fused multiply-adds).  Other orders (ascending
+    rows, or placed for shared lines) are 1.4 to 2 times further from 64 bits."""
+    m = _spiral(n, 31)
+    m = layout.reorder(m, layout.rcm_mapping(m))
+    K = m.H_init.astype(np.float32)
+    want = oracle.Port(m, "fp64").eval_rhs(K.astype(np.float64))
+    p = capi.Plain()
+    try:
+        p.init_model(m, "fp32")
+        p.select_kernel(capi.Plain.lane_shape(1, 4))
+        err = np.linalg.norm(p.eval_rhs(K).reshape(-1, 4) - want)
+    finally:
+        p.finalize()
+    assert err <= 1.25 * np.linalg.norm(oracle.Port(m, "fp32").eval_rhs(K) - want)
