@@ -317,6 +317,27 @@ struct __align__(16) NodeWork {
     double poly[kMaxK * kPolyLd];
 };
 
+// The pivot row's buffer is the parity of its column.  A lane reads it after the step's one
+// __syncwarp, so a buffer may be written again two steps on: the step between has a
+// __syncwarp that follows those reads.  Where two steps that follow each other share a
+// parity -- after the padding columns of an odd k, and from the last column of one system to
+// the first of the other -- the second starts with a __syncwarp of its own.
+__host__ __device__ constexpr bool eliminates(int p, int k) { return p < kNPoly || p >= kPolyRow || p < k; }
+__host__ __device__ constexpr bool fenced(int p) { return p == 0 || p == kPolyRow; }
+constexpr bool pivot_rows_ordered() {
+    for (int k = 1; k <= kMaxK; ++k) {
+        int before = -1;
+        for (int q = 0; q < 2 * kRhsCol; ++q) {
+            const int p = q % kRhsCol;
+            if (!eliminates(p, k)) continue;
+            if (before >= 0 && (before & 1) == (p & 1) && !fenced(p)) return false;
+            before = p;
+        }
+    }
+    return true;
+}
+static_assert(pivot_rows_ordered(), "a pivot row is overwritten while lanes may still read it");
+
 __device__ __forceinline__ void poly15(double xi, double eta, double* out) {
     int col = 0;
     for (int t = 0; t <= 4; ++t)
@@ -417,7 +438,7 @@ weights_kernel(const double* __restrict__ X, const int* __restrict__ idx, int n,
         double pval[3] = {1.0, 1.0, 1.0};     // its pivot
 #pragma unroll
         for (int p = 0; p < kRhsCol; ++p) {
-            if (p >= kNPoly && p < kPolyRow && p >= k) continue;  // padding of a narrower stencil
+            if (!eliminates(p, k)) continue;                      // padding of a narrower stencil
             const int hp = p & 1, ip = p >> 1;                    // where column p is held
             double v[3];
             unsigned key = 0;
@@ -433,6 +454,7 @@ weights_kernel(const double* __restrict__ X, const int* __restrict__ idx, int n,
             ok = ok && key >= 64u;
             const int br = 63 - (int)(key & 63u);
             double* pr = w.prow[p & 1][h];
+            if (fenced(p)) __syncwarp();
 #pragma unroll
             for (int s = 0; s < 3; ++s)
                 if (br == g + 16 * s) {
