@@ -78,10 +78,12 @@ struct EnsArgs;
 
 namespace ens {
 
-__device__ __forceinline__ float4 ldg_f4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+// State and accumulator rows are read with coherent loads, never the read-only path: the stage
+// before this one, resident beside it, or this one itself writes them.
+__device__ __forceinline__ float4 ld_f4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 // two float4 at p (32-byte aligned) in one access
-__device__ __forceinline__ void ldg_2f4(const float* p, float4 (&v)[2]) {
-    asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+__device__ __forceinline__ void ld_2f4(const float* p, float4 (&v)[2]) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[0].z), "=f"(v[0].w), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[1].z),
                    "=f"(v[1].w)
                  : "l"(p));
@@ -91,7 +93,7 @@ __device__ __forceinline__ void st_2f4(float* p, const float4 (&v)[2]) {
                  "f"(v[0].w), "f"(v[1].x), "f"(v[1].y), "f"(v[1].z), "f"(v[1].w)
                  : "memory");
 }
-__device__ __forceinline__ float2 ldg_f2(const float* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
+__device__ __forceinline__ float2 ld_f2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 
 // hi = bf16(a, b) (round to nearest even), lo = bf16 of the remainders; packed pairs, a in the low half.
 __device__ __forceinline__ uint32_t bf16x2_split(float a, float b, uint32_t& lo) {
@@ -180,7 +182,7 @@ struct Operands<T, MPC, kTf32x3> {
         float4 cen;           // centre state of the same member-fields
     };
     using Cen = float4;
-    __device__ static Cen load_cen(const float* p) { return ldg_f4(p); }
+    __device__ static Cen load_cen(const float* p) { return ld_f4(p); }
 
     __device__ static void fetch_idx(const int* rows, int gc, const Thread& th, Fetch& f) {
         f.idx = __ldg(reinterpret_cast<const int4*>(rows + gc * kEnsKc + 4 * th.kg));
@@ -293,7 +295,7 @@ struct HalfOperands {
         float2 cen;
     };
     using Cen = float2;
-    __device__ static Cen load_cen(const float* p) { return ldg_f2(p); }
+    __device__ static Cen load_cen(const float* p) { return ld_f2(p); }
 
     __device__ static void fetch_idx(const int* rows, int gc, const Thread& th, Fetch& f) {
         const int4* r = reinterpret_cast<const int4*>(rows + gc * kEnsKc + 8 * th.kh);

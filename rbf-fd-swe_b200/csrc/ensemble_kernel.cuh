@@ -462,14 +462,14 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
                 const int mfb = col0 + ch * 32 + 4 * pair_member(0);
                 const long e4 = node * a.mf + mfb, eh = node * members + (mfb >> 2);
                 auto two = [](const double* p, double (&v)[2]) {
-                    const double2 d = __ldg(reinterpret_cast<const double2*>(p));
+                    const double2 d = *reinterpret_cast<const double2*>(p);
                     v[0] = d.x; v[1] = d.y;
                 };
-                ens::ldg_2f4(a.Kin + e4, o.own);
+                ens::ld_2f4(a.Kin + e4, o.own);
                 if (MODE != kEvalOnly) two(a.Hh + eh, o.hh);
                 if (kHD) {
-                    ens::ldg_2f4(a.H32 + e4, o.h32);
-                    ens::ldg_2f4(a.D32 + e4, o.d32);
+                    ens::ld_2f4(a.H32 + e4, o.h32);
+                    ens::ld_2f4(a.D32 + e4, o.d32);
                     two(a.Dh + eh, o.dh);
                 }
             } else {
@@ -480,12 +480,12 @@ __global__ void __launch_bounds__(EnsCfg<T, MPC, PREC>::kThreads, 1) ens_stage_k
                     const int mfb = col0 + ch * 32 + 4 * pair_member(pi);
                     const long e4 = node * a.mf + mfb;
                     const long eh = node * members + (mfb >> 2);
-                    o.own[pi] = ens::ldg_f4(a.Kin + e4);
-                    if (MODE != kEvalOnly) o.hh[pi] = __ldg(a.Hh + eh);
+                    o.own[pi] = ens::ld_f4(a.Kin + e4);
+                    if (MODE != kEvalOnly) o.hh[pi] = a.Hh[eh];
                     if (kHD) {
-                        o.h32[pi] = ens::ldg_f4(a.H32 + e4);
-                        o.d32[pi] = ens::ldg_f4(a.D32 + e4);
-                        o.dh[pi] = __ldg(a.Dh + eh);
+                        o.h32[pi] = ens::ld_f4(a.H32 + e4);
+                        o.d32[pi] = ens::ld_f4(a.D32 + e4);
+                        o.dh[pi] = a.Dh[eh];
                     }
                 }
             }
