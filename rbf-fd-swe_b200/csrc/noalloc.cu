@@ -137,10 +137,11 @@ __global__ void __launch_bounds__(kRowThreads, 4) rowmajor_stage_kernel(const Ro
         if (8 * m + k < a.nnbr) row[m] = checked_neighbour(row[m], a.n, ii, 8 * m + k);
     pdl_wait();
     pdl_trigger();
+    // (coherent loads: the stage before, resident beside this one, writes these rows)
     T kv[kSlotChunks][4];
 #pragma unroll
     for (int m = 0; m < kSlotChunks; ++m)
-        if (row[m] >= 0) Quad<T>::load_row(a.Kin + 4L * row[m], kv[m]);
+        if (row[m] >= 0) Quad<T>::load_row_rw(a.Kin + 4L * row[m], kv[m]);
     // lanes 5-7: the own state and the H and D rows
     if (k == 5 || (kHD && k > 5)) {
         T r[4];

@@ -109,20 +109,14 @@ __device__ __forceinline__ void points(const T* PTl, long tile, int t, T (&pt)[k
 #pragma unroll
     for (int f = 0; f < kPointFields; ++f) pt[f] = __ldg(p + f * kLaneTile);
 }
-// one state row (u, v, w, h): a whole 32-byte sector in one load (FP64)
+// one state row (u, v, w, h): a whole 32-byte sector in one load (FP64).  A coherent load: the
+// stage before, resident beside this one, or this one itself writes the row.
 __device__ __forceinline__ void state_row(const double* p, double (&v)[4]) {
-    asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-                 : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
-                 : "l"(p));
-}
-__device__ __forceinline__ void state_row(const float* p, float (&v)[4]) { Quad<float>::load_row(p, v); }
-// the same for rows that this kernel writes, and the store
-__device__ __forceinline__ void own_row(const double* p, double (&v)[4]) {
     asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
                  : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
                  : "l"(p));
 }
-__device__ __forceinline__ void own_row(const float* p, float (&v)[4]) { Quad<float>::load_row_rw(p, v); }
+__device__ __forceinline__ void state_row(const float* p, float (&v)[4]) { Quad<float>::load_row_rw(p, v); }
 __device__ __forceinline__ void put_row(double* p, const double (&v)[4]) {
     asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3]) : "memory");
 }
@@ -236,8 +230,8 @@ __global__ void __launch_bounds__(kLaneThreads, MINB) stage_lane_kernel(const La
         lane::put_row(a.Kout + 4 * i, kn);
     } else {
         T h[4], d[4];
-        lane::own_row(a.H + 4 * i, h);
-        lane::own_row(a.D + 4 * i, d);
+        lane::state_row(a.H + 4 * i, h);
+        lane::state_row(a.D + 4 * i, d);
         if (MODE == kStage1 || MODE == kStage2) {
             // update_D(D, F, 2) and eval_K(H, K, F, c)
             T kn[4];

@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(TmaShape<TILE>::kThreads, TmaShape<TILE>::kCta
         const int nbr[4] = {nb.x, nb.y, nb.z, nb.w};
         T kg[kSlotChunks][4];
 #pragma unroll
-        for (int m = 0; m < kSlotChunks; ++m) Quad<T>::load_row(a.Kin + 4L * nbr[m], kg[m]);
+        for (int m = 0; m < kSlotChunks; ++m) Quad<T>::load_row_rw(a.Kin + 4L * nbr[m], kg[m]);
         T acc[16];
 #pragma unroll
         for (int q = 0; q < 16; ++q) acc[q] = T(0);
