@@ -226,6 +226,13 @@ int swe_gen_weights(int n, int k, const double* X, const int* idx, double* D);
  * limit_s (0 < limit_s <= 2), with the context still usable.  waited_s (may
  * be NULL) receives the time the kernel waited. */
 int swe_selftest_wait_timeout(double limit_s, double* waited_s);
+/* The same for the waits between the blocks of the plain form's resident step kernel:
+ * launches (on the plain form's stream, asynchronous) one block that waits at most
+ * limit_s (0 < limit_s <= 2) for a second one that was never launched.  From then on
+ * swe_cuda_sync, swe_cuda_get_state and swe_cuda_invariants return SWE_ERR_TIMEOUT, as
+ * after a step whose wait ran out, until swe_cuda_init is called again.
+ * SWE_ERR_STATE where no resident kernel is set up. */
+int swe_selftest_step_wait(double limit_s);
 
 /* ---------------------------------------------------------------------------
  * Batched-ensemble form (members share one grid; tcgen05 tensor cores)

@@ -459,26 +459,27 @@ static int upload_static(Plain& P, const void* x, const void* y, const void* z, 
     return SWE_OK;
 }
 
-// Reads the pipelined kernel's bounded-wait error word: enqueues its copy into
-// pinned memory and synchronises the stream once (callers that also read data
-// back enqueue their copy first, so one synchronisation serves both).
-static int check_tma_err() {
+// Synchronises the stream and reports a bounded wait that ran out: the resident kernel's flag
+// (in pinned memory, whatever kernel is selected by now) and the pipelined kernel's error word,
+// whose copy into pinned memory is enqueued first (callers that also read data back enqueue
+// their copy before that, so one synchronisation serves all).  Every call that answers from
+// the stepped state ends here.
+static int check_waits() {
     Plain& P = g_plain;
-    if (P.res_failed && P.res_lpn) {
-        SWE_CUDA_TRY(cudaStreamSynchronize(P.stream));
-        if (*(volatile int*)P.res_failed) {
-            set_error("resident step kernel: a bounded wait for another block ran out");
-            return SWE_ERR_TIMEOUT;
-        }
-    }
+    auto resident = [&]() {
+        if (!P.res_failed || !*(volatile int*)P.res_failed) return SWE_OK;
+        set_error("resident step kernel: a bounded wait for another block ran out");
+        return (int)SWE_ERR_TIMEOUT;
+    };
     // only the pipelined kernel writes the word: read it back (one more small copy before
     // the synchronisation) only after such a launch
     if (!P.err || !P.err_host || !P.err_pending) {
         SWE_CUDA_TRY(cudaStreamSynchronize(P.stream));
-        return SWE_OK;
+        return resident();
     }
     SWE_CUDA_TRY(cudaMemcpyAsync(P.err_host, P.err, sizeof(int), cudaMemcpyDeviceToHost, P.stream));
     SWE_CUDA_TRY(cudaStreamSynchronize(P.stream));
+    SWE_TRY(resident());
     const int h = *P.err_host;
     P.err_pending = h != 0;   // a timeout stays reported until the word is cleared
     if (h) {
@@ -658,7 +659,7 @@ int swe_cuda_init(int fsize, int layout, int simd_length, int compute_size, int 
         for (int k = 1; k < 3; ++k)
             if (P.tune_us[k] < P.tune_us[best]) best = k;
         P.kernel_choice = best;
-        SWE_TRY(check_tma_err());
+        SWE_TRY(check_waits());
         // Whole steps in the resident kernel where it is faster than four launches of the
         // stage kernel, with the stage kernel's lanes per node (a step and its four substeps
         // give the same bits): 2 or 4, whichever of those whose stage kernel is within 10 % of
@@ -692,7 +693,7 @@ int swe_cuda_init(int fsize, int layout, int simd_length, int compute_size, int 
                     SWE_CUDA_TRY(cudaEventSynchronize(e1));
                     SWE_CUDA_TRY(cudaEventElapsedTime(&ms[r & 1], e0, e1));
                 }
-                SWE_TRY(check_tma_err());
+                SWE_TRY(check_waits());
                 const float step = (ms[1] - ms[0]) * 1e3f / 8.f;
                 if (step < step_best) {
                     step_best = step;
@@ -747,7 +748,7 @@ int swe_cuda_get_state(void* Hh) {
         SWE_TRY(permute_state(P.H, P.raw, 1));
         SWE_CUDA_TRY(cudaMemcpyAsync(Hh, P.raw, bytes, cudaMemcpyDeviceToHost, P.stream));
     }
-    return check_tma_err();   // one synchronisation covers the state copy and the error word
+    return check_waits();   // one synchronisation covers the state copy and the error word
 }
 
 int swe_cuda_eval_rhs(const void* K, void* Fh) {
@@ -896,7 +897,7 @@ int swe_cuda_halo_unpack(int substep_id, const void* recv_buf) {
 
 int swe_cuda_sync(void) {
     SWE_TRY(require_ready());
-    return check_tma_err();   // synchronises the stream
+    return check_waits();   // synchronises the stream
 }
 
 int swe_cuda_select_kernel(int which) {
@@ -1004,7 +1005,7 @@ int swe_cuda_invariants(double* me) {
     count_launch();
     SWE_CUDA_TRY(cudaGetLastError());
     SWE_CUDA_TRY(cudaMemcpyAsync(me, P.inv, 2 * sizeof(double), cudaMemcpyDeviceToHost, P.stream));
-    SWE_CUDA_TRY(cudaStreamSynchronize(P.stream));
+    SWE_TRY(check_waits());
     const double area = 4.0 * 3.14159265358979323846 / (double)P.n;
     me[0] *= area;
     me[1] *= area;
@@ -1037,6 +1038,22 @@ int swe_hist_stats(long long* out) {
     out[1] = g_plain.hist.records();
     out[2] = g_plain.hist.bytes();
     out[3] = g_plain.steps_done;
+    return SWE_OK;
+}
+
+int swe_selftest_step_wait(double limit_s) {
+    SWE_TRY(require_ready());
+    Plain& P = g_plain;
+    if (!(limit_s > 0.0) || limit_s > 2.0) { set_error("swe_selftest_step_wait: limit must be in (0, 2] seconds"); return SWE_ERR_ARG; }
+    if (!P.res_sync) { set_error("swe_selftest_step_wait: the resident kernel is not set up"); return SWE_ERR_STATE; }
+    res::Args<double> a{};
+    a.counter = P.res_sync;
+    a.failed = P.res_failed;
+    a.wait_ns = (unsigned long long)(limit_s * 1e9);
+    SWE_CUDA_TRY(cudaMemsetAsync(P.res_sync, 0, res::kSyncWords * sizeof(unsigned), P.stream));
+    res::lone_block_kernel<<<1, 32, 0, P.stream>>>(a);
+    count_launch();
+    SWE_CUDA_TRY(cudaGetLastError());
     return SWE_OK;
 }
 

@@ -48,6 +48,7 @@ struct Args {
     double dt6;
     unsigned* counter;                 // arrivals of the CTAs, zero at launch; abort word 32 words on
     int* failed;                       // set when a wait ran out (pinned host or device memory)
+    unsigned long long wait_ns = kWaitNs;
 };
 
 // Static data as swe_cuda_init packs it.
@@ -142,7 +143,7 @@ __device__ __forceinline__ bool exchange(const Args<T>& a, unsigned stage, int* 
                 unsigned long long t;
                 asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
                 if (t0 == 0) t0 = t;
-                if (*abort_word != 0 || t - t0 > (stage == 1 ? kFirstWaitNs : kWaitNs)) {
+                if (*abort_word != 0 || t - t0 > (stage == 1 ? kFirstWaitNs : a.wait_ns)) {
                     *abort_word = 1;
                     *(volatile int*)a.failed = 1;
                     __threadfence_system();
@@ -155,6 +156,13 @@ __device__ __forceinline__ bool exchange(const Args<T>& a, unsigned stage, int* 
     }
     __syncthreads();
     return *s_ok != 0;
+}
+
+// One block that waits, as after a step's second stage, for a block that was never launched:
+// the path of a wait that runs out, without anything to run out of (swe_selftest_step_wait).
+static __global__ void lone_block_kernel(Args<double> a) {
+    __shared__ int ok;
+    exchange(a, 2, &ok);
 }
 
 template <typename T, int LPN, int THREADS, class Src, bool STREAM>
