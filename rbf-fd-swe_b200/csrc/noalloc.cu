@@ -294,7 +294,7 @@ bool run_resident(const RowMajorArgs<T>& r, T* Ka, T* Kb, T dt, int nsteps, cons
     a.counter = A.sync;
     a.failed = A.failed;
     const RowMajor<T> src{r.idx, r.Dx, r.Dy, r.Dz, r.L, r.x, r.y, r.z, r.f, r.ghm, r.pu, r.pv, r.pw, r.gg};
-    e = lpn == 4 ? res::launch<T, 4>(a, src, ctas, smem, false, stream) : res::launch<T, 2>(a, src, ctas, smem, false, stream);
+    e = lpn == 4 ? res::launch<T, 4>(a, src, ctas, smem, A.smem, false, stream) : res::launch<T, 2>(a, src, ctas, smem, A.smem, false, stream);
     if (e == cudaErrorCooperativeLaunchTooLarge) {      // fewer SMs for this stream than the device has
         cudaGetLastError();
         return false;

@@ -128,7 +128,7 @@ struct Plain {
 
     // resident multi-step kernel (resident.cuh): lanes per node, 0 where it is not in use
     int res_lpn = 0, res_m = 0, res_ctas = 0, res_min_steps = 1;
-    size_t res_smem = 0;
+    size_t res_smem = 0, res_smem_max = 0;
     bool res_stream = false;        // it streams part of the weights
     unsigned* res_sync = nullptr;
     int* res_failed = nullptr;      // pinned: a bounded wait ran out
@@ -354,8 +354,8 @@ struct Plain {
         a.failed = res_failed;
         const T* wl = reinterpret_cast<const T*>(Wl);
         const T* pt = reinterpret_cast<const T*>(PTl);
-        if (idxs_fit) return res::launch<T, LPN>(a, res::Packed<T, true>{wl, idxl, idxs, pt}, res_ctas, res_smem, res_stream, stream);
-        return res::launch<T, LPN>(a, res::Packed<T, false>{wl, idxl, idxs, pt}, res_ctas, res_smem, res_stream, stream);
+        if (idxs_fit) return res::launch<T, LPN>(a, res::Packed<T, true>{wl, idxl, idxs, pt}, res_ctas, res_smem, res_smem_max, res_stream, stream);
+        return res::launch<T, LPN>(a, res::Packed<T, false>{wl, idxl, idxs, pt}, res_ctas, res_smem, res_smem_max, res_stream, stream);
     }
     cudaError_t launch_resident(int nsteps) {
         count_launch();
@@ -365,10 +365,10 @@ struct Plain {
     // Splits the grid over the SMs for lpn lanes a node (fits: false where it does not).
     int setup_resident(int lpn, bool& fits) {
         int nsm = 0;
-        size_t most = 0;
-        SWE_CUDA_TRY(res::smem_limit(nsm, most));
-        fits = fsize == 8 ? res::split<double>(n, nnbr, lpn, nsm, most, true, res_m, res_ctas, res_smem, res_stream)
-                          : res::split<float>(n, nnbr, lpn, nsm, most, true, res_m, res_ctas, res_smem, res_stream);
+        SWE_CUDA_TRY(res::smem_limit(nsm, res_smem_max));
+        fits = fsize == 8
+                   ? res::split<double>(n, nnbr, lpn, nsm, res_smem_max, true, res_m, res_ctas, res_smem, res_stream)
+                   : res::split<float>(n, nnbr, lpn, nsm, res_smem_max, true, res_m, res_ctas, res_smem, res_stream);
         res_lpn = fits ? lpn : 0;
         if (!fits) return SWE_OK;
         if (!res_sync) {

@@ -386,11 +386,14 @@ inline bool split(int n, int nnbr, int lpn, int sms, size_t smem_max, bool strea
 }
 
 template <typename T, int LPN, class Src>
-inline cudaError_t launch(const Args<T>& a, const Src& src, int ctas, size_t smem, bool stream, cudaStream_t st) {
+inline cudaError_t launch(const Args<T>& a, const Src& src, int ctas, size_t smem, size_t smem_max, bool stream,
+                          cudaStream_t st) {
     auto kernel = a.m * LPN <= kFew ? steps_kernel<T, LPN, kFew, Src, false> : steps_kernel<T, LPN, kMost, Src, false>;
     if constexpr (Src::kNodeFast && sizeof(T) == 8 && LPN == 2)
         if (stream) kernel = steps_kernel<T, LPN, kMost, Src, true>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the device's limit in every call, never the call's own size: another thread may be
+    // between its attribute and its launch
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(a.counter, 0, kSyncWords * sizeof(unsigned), st);
     if (e != cudaSuccess) return e;

@@ -191,3 +191,45 @@ def test_noalloc_calls_can_be_captured(n):
     torch.cuda.synchronize()
     assert torch.equal(H, want)
     del g
+
+
+def test_noalloc_calls_from_two_threads_do_not_disturb_each_other():
+    """Two threads issue calls of different sizes at once, as callers that order them on the GPU
+    by events do.  Each thread captures and instantiates its calls, so that none runs: a launch
+    whose shared memory the other thread lowered would be refused."""
+    import threading
+    import torch
+
+    cu = ctypes.CDLL("libcuda.so.1")
+    vp = ctypes.c_void_p
+    models = [_spiral(n, 31) for n in (5000, 18000)]
+    arrays = [_device_arrays(m, "fp64") for m in models]
+    states = [torch.from_numpy(m.H_init).cuda() for m in models]
+    for m, t, H in zip(models, arrays, states):                # first calls, outside capture
+        _call(m, "fp64", 2, H, torch.cuda.current_stream().cuda_stream, t)
+    torch.cuda.synchronize()
+    errors = []
+
+    def issue(m, t, H):
+        try:
+            torch.cuda.set_device(0)
+            stream = torch.cuda.Stream()
+            for _ in range(400):
+                graph, executable = vp(), vp()
+                assert cu.cuStreamBeginCapture_v2(vp(stream.cuda_stream), 1) == 0
+                try:
+                    _call(m, "fp64", 2, H, stream.cuda_stream, t)
+                finally:
+                    assert cu.cuStreamEndCapture(vp(stream.cuda_stream), ctypes.byref(graph)) == 0
+                assert cu.cuGraphInstantiateWithFlags(ctypes.byref(executable), graph, ctypes.c_ulonglong(0)) == 0
+                cu.cuGraphExecDestroy(executable)
+                cu.cuGraphDestroy(graph)
+        except Exception as e:                                  # noqa: BLE001 (reported by the main thread)
+            errors.append(e)
+
+    threads = [threading.Thread(target=issue, args=a) for a in zip(models, arrays, states)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not errors, errors[0]
