@@ -153,6 +153,15 @@ int swe_cuda_sync(void);
  * prefetch when s >= 15. */
 int swe_cuda_select_kernel(int which);
 int swe_cuda_kernel_info(int* info);
+/* The resident kernel of swe_cuda_step: info[4] = {lanes per node (0: whole steps run as
+ * stage launches), part of the weights streamed from L2 in every stage (0/1), steps a call
+ * must have to use it, blocks}.  swe_cuda_select_step_kernel replaces swe_cuda_init's choice:
+ * 0 = stage launches, 2 / 4 = the resident kernel with that many lanes per node for calls of
+ * any number of steps, and kernel 2 with as many for substeps (the same bits); SWE_ERR_ARG
+ * where the patch has halo rows or does not fit.  swe_cuda_select_kernel also ends the
+ * resident kernel's use. */
+int swe_cuda_step_kernel_info(int* info);
+int swe_cuda_select_step_kernel(int lanes);
 /* Index width of kernel 2's gather rows: 16 (the default whenever every stencil
  * row lies within 32767 rows of its node; SWE_ERR_ARG otherwise) or 32.  The
  * results are the same bits either way; 16 halves the index bytes. */

@@ -957,6 +957,46 @@ int swe_cuda_kernel_info(int* out) {
     return SWE_OK;
 }
 
+int swe_cuda_select_step_kernel(int lanes) {
+    SWE_TRY(require_ready());
+    if (lanes != 0 && lanes != 2 && lanes != 4) {
+        set_error("swe_cuda_select_step_kernel: 0 (stage launches), 2 or 4 lanes per node, got %d", lanes);
+        return SWE_ERR_ARG;
+    }
+    Plain& P = g_plain;
+    SWE_CUDA_TRY(cudaStreamSynchronize(P.stream));
+    if (lanes == 0) {
+        P.res_lpn = 0;
+        return SWE_OK;
+    }
+    const int before = P.res_lpn;
+    bool fits = false;
+    if (P.pid0 == 0 && P.rows == P.n) SWE_TRY(P.setup_resident(lanes, fits));
+    if (!fits) {
+        set_error("swe_cuda_select_step_kernel: %s", P.rows != P.n ? "a patch with halo rows steps by swe_cuda_rk_substep"
+                                                                    : "the patch does not fit the SMs' shared memory");
+        if (before) SWE_TRY(P.setup_resident(before, fits));
+        return SWE_ERR_ARG;
+    }
+    P.res_min_steps = 1;
+    P.kernel_choice = 2;          // the stage kernel with the same lanes: the same bits
+    P.lane_lpn = lanes;
+    if (P.graph) cudaGraphExecDestroy(P.graph);
+    P.graph = nullptr;
+    return P.build_graph();
+}
+
+int swe_cuda_step_kernel_info(int* out) {
+    SWE_TRY(require_ready());
+    if (!out) { set_error("null out"); return SWE_ERR_ARG; }
+    const Plain& P = g_plain;
+    out[0] = P.res_lpn;
+    out[1] = P.res_lpn && P.res_stream ? 1 : 0;
+    out[2] = P.res_lpn ? P.res_min_steps : 0;
+    out[3] = P.res_lpn ? P.res_ctas : 0;
+    return SWE_OK;
+}
+
 int swe_cuda_set_timing(int enabled) {
     SWE_TRY(require_ready());
     Plain& P = g_plain;

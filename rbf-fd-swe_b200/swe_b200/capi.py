@@ -74,6 +74,8 @@ def load() -> ctypes.CDLL:
     lib.swe_cuda_stream.restype = vp
     lib.swe_cuda_select_kernel.argtypes = [i]
     lib.swe_cuda_kernel_info.argtypes = [vp]
+    lib.swe_cuda_step_kernel_info.argtypes = [vp]
+    lib.swe_cuda_select_step_kernel.argtypes = [i]
     lib.swe_cuda_set_index_width.argtypes = [i]
     lib.swe_hist_open.argtypes = [ctypes.c_char_p, i]
     lib.swe_gen_stencils.argtypes = [i, i, vp, vp]
@@ -270,6 +272,17 @@ class Plain:
                 "pipelined_tile": int(out[1]), "lanes_per_node": int(out[4]), "l2_prefetch": bool(out[6]),
                 "ctas_per_sm": int(out[7]), "index_offsets_16bit": bool(out[8]),
                 "tune_us": {"pipelined": out[2] / 1e3, "register": out[3] / 1e3, "lane": out[5] / 1e3}}
+
+    def select_step_kernel(self, lanes: int) -> None:
+        """step() as stage launches (0), or in the resident kernel with 2 or 4 lanes per node."""
+        check("swe_cuda_select_step_kernel", self.lib.swe_cuda_select_step_kernel(int(lanes)))
+
+    def step_kernel_info(self) -> dict:
+        """The resident kernel of step(): lanes per node (0: not in use), whether it streams part
+        of the weights, the steps a call must have to use it, its blocks."""
+        out = np.zeros(4, dtype=np.int32)
+        check("swe_cuda_step_kernel_info", self.lib.swe_cuda_step_kernel_info(_p(out)))
+        return {"lanes_per_node": int(out[0]), "streamed": bool(out[1]), "min_steps": int(out[2]), "blocks": int(out[3])}
 
     def invariants(self) -> np.ndarray:
         """FP64 (mass, energy); raises SweError (SWE_ERR_NONFINITE) when the state holds NaN/Inf."""

@@ -54,3 +54,80 @@ def test_fp32_rhs_of_one_lane_per_node_is_as_exact_as_the_restatement(n):
     finally:
         p.finalize()
     assert err <= 1.25 * np.linalg.norm(oracle.Port(m, "fp32").eval_rhs(K) - want)
+
+
+# lanes per node and whether the weights are streamed, at sizes around the splits' edges (148 SMs,
+# 31 neighbours: 2 lanes hold 27,232 nodes in FP64 and stream to 42,624; nodes per block in
+# multiples of 8, streamed of 32)
+@pytest.mark.parametrize("prec,n,nnbr,lanes,streamed", [
+    ("fp64", 149, 31, 4, False), ("fp64", 9731, 28, 4, False), ("fp64", 10242, 31, 2, False), ("fp64", 27232, 31, 2, False),
+    ("fp64", 27233, 31, 2, True), ("fp64", 35009, 25, 2, True), ("fp64", 37889, 31, 2, True), ("fp64", 42624, 32, 2, True),
+    ("fp32", 1185, 31, 2, False), ("fp32", 20001, 32, 4, False), ("fp32", 47360, 17, 2, False)])
+def test_whole_steps_in_the_resident_kernel_equal_substeps(prec, n, nnbr, lanes, streamed):
+    """The resident kernel, selected: a call is one launch and gives the bits of the stage
+    launches of as many substeps; stage launches when they are selected again."""
+    m = _spiral(n, nnbr)
+    m = layout.reorder(m, layout.rcm_mapping(m))
+    H0 = m.H_init.astype(np.float64 if prec == "fp64" else np.float32)
+    p = capi.Plain()
+    try:
+        p.init_model(m, prec)
+        p.select_step_kernel(lanes)
+        info = p.step_kernel_info()
+        assert (info["lanes_per_node"], info["streamed"], info["min_steps"]) == (lanes, streamed, 1)
+        for steps in (1, 7):
+            p.set_state(H0)
+            before = capi.kernel_launches()
+            p.step(steps)
+            assert capi.kernel_launches() - before == 1
+            got = p.get_state()
+            p.set_state(H0)
+            for _ in range(steps):
+                for s in range(4):
+                    p.rk_substep(s)
+            assert np.array_equal(got, p.get_state()), steps
+        p.select_step_kernel(0)
+        assert p.step_kernel_info()["lanes_per_node"] == 0
+        p.set_state(H0)
+        before = capi.kernel_launches()
+        p.step(7)
+        assert capi.kernel_launches() - before == 28
+        assert np.array_equal(got, p.get_state())
+    finally:
+        p.finalize()
+
+
+def test_step_kernel_selection_refuses_what_does_not_fit():
+    m = _spiral(25001, 31)
+    p = capi.Plain()
+    try:
+        p.init_model(m, "fp64")
+        p.select_step_kernel(2)
+        for lanes in (1, 3, 4):                     # 4 lanes a node: more threads than a block has
+            with pytest.raises(capi.SweError) as e:
+                p.select_step_kernel(lanes)
+            assert capi.STATUS[e.value.status] == "SWE_ERR_ARG"
+            assert p.step_kernel_info()["lanes_per_node"] == 2
+    finally:
+        p.finalize()
+
+
+def test_init_chooses_the_resident_kernel():
+    """swe_cuda_init chooses by timing: 40,001 nodes in FP32, clearly faster resident (4.2 against 4.7 us
+    a stage), in one of three tries."""
+    m = _spiral(40001, 31)
+    m = layout.reorder(m, layout.rcm_mapping(m))
+    p = capi.Plain()
+    try:
+        for _ in range(3):
+            p.init_model(m, "fp32")
+            if p.step_kernel_info()["lanes_per_node"]:
+                break
+        info = p.step_kernel_info()
+        assert info["lanes_per_node"]
+        p.set_state(m.H_init.astype(np.float32))
+        before = capi.kernel_launches()
+        p.step(max(20, info["min_steps"]))
+        assert capi.kernel_launches() - before == 1
+    finally:
+        p.finalize()
