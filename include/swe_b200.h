@@ -162,7 +162,7 @@ int swe_cuda_kernel_info(int* info);
  * resident kernel's use. */
 int swe_cuda_step_kernel_info(int* info);
 int swe_cuda_select_step_kernel(int lanes);
-/* Index width of kernel 2's gather rows: 16 (the default whenever every stencil
+/* Index width of kernel 2's and the resident kernel's gather rows: 16 (the default whenever every stencil
  * row lies within 32767 rows of its node; SWE_ERR_ARG otherwise) or 32.  The
  * results are the same bits either way; 16 halves the index bytes. */
 int swe_cuda_set_index_width(int bits);

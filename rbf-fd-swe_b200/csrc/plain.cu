@@ -354,7 +354,7 @@ struct Plain {
         a.failed = res_failed;
         const T* wl = reinterpret_cast<const T*>(Wl);
         const T* pt = reinterpret_cast<const T*>(PTl);
-        if (idxs_fit) return res::launch<T, LPN>(a, res::Packed<T, true>{wl, idxl, idxs, pt}, res_ctas, res_smem, res_smem_max, res_stream, stream);
+        if (idxs_ok) return res::launch<T, LPN>(a, res::Packed<T, true>{wl, idxl, idxs, pt}, res_ctas, res_smem, res_smem_max, res_stream, stream);
         return res::launch<T, LPN>(a, res::Packed<T, false>{wl, idxl, idxs, pt}, res_ctas, res_smem, res_smem_max, res_stream, stream);
     }
     cudaError_t launch_resident(int nsteps) {

@@ -97,6 +97,30 @@ def test_whole_steps_in_the_resident_kernel_equal_substeps(prec, n, nnbr, lanes,
         p.finalize()
 
 
+@pytest.mark.parametrize("prec,n,lanes", [("fp64", 10242, 2), ("fp64", 10242, 4), ("fp64", 35009, 2), ("fp32", 20001, 4)])
+def test_resident_rows_of_both_widths(prec, n, lanes):
+    """swe_cuda_set_index_width holds for the resident kernel too (its 32-bit rows took no part
+    before on grids whose rows fit 16 bits): the same bits."""
+    m = _spiral(n, 31)
+    m = layout.reorder(m, layout.rcm_mapping(m))
+    H0 = m.H_init.astype(np.float64 if prec == "fp64" else np.float32)
+    p = capi.Plain()
+    try:
+        p.init_model(m, prec)
+        p.select_step_kernel(lanes)
+        assert p.kernel_info()["index_offsets_16bit"]
+        got = []
+        for bits in (16, 32):
+            p.set_index_width(bits)
+            assert p.step_kernel_info()["lanes_per_node"] == lanes
+            p.set_state(H0)
+            p.step(7)
+            got.append(p.get_state())
+        assert np.array_equal(*got)
+    finally:
+        p.finalize()
+
+
 def test_step_kernel_selection_refuses_what_does_not_fit():
     m = _spiral(25001, 31)
     p = capi.Plain()
