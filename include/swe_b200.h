@@ -117,7 +117,11 @@ int swe_cuda_halo_unpack(int substep_id, const void* recv_buf);
 /* nsteps full RK4 steps (4 stages each) from a captured CUDA graph, or, where
  * swe_cuda_init found it faster (grids whose static data fits in the SMs' shared
  * memory; no history output open; no kernel forced by swe_cuda_select_kernel), in
- * one kernel that holds all SMs for the steps; the same bits either way.
+ * kernels of up to 200 steps with a block for every SM; the same bits either way.
+ * Kernels of other streams that hold some SMs do not keep the steps from running (on
+ * the SMs that are left); one that holds a part of every SM does until it ends, and a
+ * program whose such kernel waits for the steps selects stage launches
+ * (swe_cuda_select_step_kernel).
  * Asynchronous; requires compute_pid_s == 0 and patch_size == compute_size
  * (no halo rows: a patch with halo rows steps by swe_cuda_rk_substep with
  * halo exchanges between substeps). */
@@ -242,6 +246,10 @@ int swe_selftest_wait_timeout(double limit_s, double* waited_s);
  * after a step whose wait ran out, until swe_cuda_init is called again.
  * SWE_ERR_STATE where no resident kernel is set up. */
 int swe_selftest_step_wait(double limit_s);
+/* Launches, on `stream` (a cudaStream_t), `blocks` blocks that take an SM's shared memory
+ * each and end after limit_s (0 < limit_s <= 2): another stream's long-lived kernel, for
+ * tests of steps that run beside one. */
+int swe_selftest_hold_sms(int blocks, double limit_s, void* stream);
 
 /* ---------------------------------------------------------------------------
  * Batched-ensemble form (members share one grid; tcgen05 tensor cores)
@@ -377,7 +385,8 @@ int swe_srv_test_withhold(int request, int stage_index);
  * and must be serialised by the caller.  Kernels go to `stream` (a
  * cudaStream_t, NULL for the default stream); the call returns once they are
  * enqueued.  Grids of a few thousand nodes or more whose static data fits in the
- * SMs' shared memory step in one kernel that holds all SMs.  Every idx entry
+ * SMs' shared memory step in kernels of up to 200 steps with a block for every SM
+ * (beside other streams' kernels as swe_cuda_step's).  Every idx entry
  * must lie in 0..n-1.  The kernels check each one as they gather: an entry outside that range is never dereferenced (the node's
  * own row is read in its place, so that call's results are wrong) and the
  * first one is recorded.  A call with nsteps = 0 steps nothing: it waits for

@@ -29,6 +29,7 @@
 // SWE_ERR_INDEX and clears it.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
@@ -283,23 +284,23 @@ bool run_resident(const RowMajorArgs<T>& r, T* Ka, T* Kb, T dt, int nsteps, cons
     a.n = r.n;
     a.nnbr = r.nnbr;
     a.m = m;
-    a.nsteps = nsteps;
     a.H = r.H;
     a.Ka = Ka;
     a.Kb = Kb;
+    a.D = r.D;
     a.gh0 = r.gh0;
     a.c01 = (T)(dt / 2.0);
     a.c2 = dt;
     a.dt6 = r.dt6;
-    a.counter = A.sync;
+    a.sync = A.sync;
     a.failed = A.failed;
     const RowMajor<T> src{r.idx, r.Dx, r.Dy, r.Dz, r.L, r.x, r.y, r.z, r.f, r.ghm, r.pu, r.pv, r.pw, r.gg};
-    e = lpn == 4 ? res::launch<T, 4>(a, src, ctas, smem, A.smem, false, stream) : res::launch<T, 2>(a, src, ctas, smem, A.smem, false, stream);
-    if (e == cudaErrorCooperativeLaunchTooLarge) {      // fewer SMs for this stream than the device has
-        cudaGetLastError();
-        return false;
+    for (int left = nsteps; left > 0 && e == cudaSuccess; left -= a.nsteps) {
+        a.nsteps = std::min(left, res::kLaunchSteps);
+        e = lpn == 4 ? res::launch<T, 4>(a, src, ctas, smem, A.smem, false, stream)
+                     : res::launch<T, 2>(a, src, ctas, smem, A.smem, false, stream);
+        count_launch();
     }
-    count_launch();
     return true;
 }
 

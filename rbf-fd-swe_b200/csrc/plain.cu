@@ -345,12 +345,13 @@ struct Plain {
         a.H = reinterpret_cast<T*>(H);
         a.Ka = reinterpret_cast<T*>(Ka);
         a.Kb = reinterpret_cast<T*>(Kb);
+        a.D = reinterpret_cast<T*>(D);
         a.gh0 = (T)gh0;
         const T dtT = (T)dt;
         a.c01 = (T)(dtT / 2.0);
         a.c2 = dtT;
         a.dt6 = (double)dtT / 6.0;
-        a.counter = res_sync;
+        a.sync = res_sync;
         a.failed = res_failed;
         const T* wl = reinterpret_cast<const T*>(Wl);
         const T* pt = reinterpret_cast<const T*>(PTl);
@@ -358,7 +359,7 @@ struct Plain {
         return res::launch<T, LPN>(a, res::Packed<T, false>{wl, idxl, idxs, pt}, res_ctas, res_smem, res_smem_max, res_stream, stream);
     }
     cudaError_t launch_resident(int nsteps) {
-        count_launch();
+        count_launch(res_stream ? 2 : 1);
         if (fsize == 8) return res_lpn == 4 ? launch_resident_t<double, 4>(nsteps) : launch_resident_t<double, 2>(nsteps);
         return res_lpn == 4 ? launch_resident_t<float, 4>(nsteps) : launch_resident_t<float, 2>(nsteps);
     }
@@ -682,10 +683,6 @@ int swe_cuda_init(int fsize, int layout, int simd_length, int compute_size, int 
                 SWE_TRY(P.setup_resident(1 << l, fits));
                 if (!fits) continue;
                 float ms[2] = {0.f, 0.f};
-                if (P.launch_resident(2) != cudaSuccess) {             // not enough SMs at once here
-                    cudaGetLastError();
-                    continue;
-                }
                 for (int r = 0; r < 4; ++r) {              // 2 and 10 steps, the first pair to warm up
                     SWE_CUDA_TRY(cudaEventRecord(e0, P.stream));
                     SWE_CUDA_TRY(P.launch_resident(r & 1 ? 10 : 2));
@@ -693,7 +690,11 @@ int swe_cuda_init(int fsize, int layout, int simd_length, int compute_size, int 
                     SWE_CUDA_TRY(cudaEventSynchronize(e1));
                     SWE_CUDA_TRY(cudaEventElapsedTime(&ms[r & 1], e0, e1));
                 }
-                SWE_TRY(check_waits());
+                SWE_CUDA_TRY(cudaStreamSynchronize(P.stream));
+                if (*(volatile int*)P.res_failed) {                    // no choice here
+                    *P.res_failed = 0;
+                    continue;
+                }
                 const float step = (ms[1] - ms[0]) * 1e3f / 8.f;
                 if (step < step_best) {
                     step_best = step;
@@ -796,8 +797,7 @@ int swe_cuda_step(int nsteps) {
     if (P.use_tma()) P.err_pending = true;
     int s = 0;
     if (P.res_lpn && !P.hist.active() && nsteps >= P.res_min_steps) {
-        constexpr int kMost = 1000;          // steps per launch: a kernel of tens of milliseconds
-        for (; s < nsteps; s += std::min(kMost, nsteps - s)) SWE_CUDA_TRY(P.launch_resident(std::min(kMost, nsteps - s)));
+        for (; s < nsteps; s += res::kLaunchSteps) SWE_CUDA_TRY(P.launch_resident(std::min(res::kLaunchSteps, nsteps - s)));
         P.steps_done += nsteps;
         s = nsteps;
     }
@@ -1087,7 +1087,7 @@ int swe_selftest_step_wait(double limit_s) {
     if (!(limit_s > 0.0) || limit_s > 2.0) { set_error("swe_selftest_step_wait: limit must be in (0, 2] seconds"); return SWE_ERR_ARG; }
     if (!P.res_sync) { set_error("swe_selftest_step_wait: the resident kernel is not set up"); return SWE_ERR_STATE; }
     res::Args<double> a{};
-    a.counter = P.res_sync;
+    a.sync = P.res_sync;
     a.failed = P.res_failed;
     a.wait_ns = (unsigned long long)(limit_s * 1e9);
     SWE_CUDA_TRY(cudaMemsetAsync(P.res_sync, 0, res::kSyncWords * sizeof(unsigned), P.stream));

@@ -2,7 +2,7 @@
 //
 // On a grid of some thousand to some ten thousand nodes a stage takes a few
 // microseconds, most of it the launch of the next kernel and chained L2 reads.  Here
-// one cooperative launch runs all steps: CTA c (one per SM) owns nodes [c m, c m + m),
+// one launch runs all steps: CTA c (one per SM) owns nodes [c m, c m + m),
 // keeps their stencil weights, pointwise records, base state and RK accumulator in
 // shared memory and their gather rows in registers, and exchanges only the stage
 // states through L2.  A stage is the node-per-lane kernel's work split (LPN lanes a
@@ -14,8 +14,16 @@
 // shared lines and 1.3-1.5 with a line per CTA and waits for the neighbours only.  K rows
 // are read with plain loads, cached in L1: the acquire makes the rows that other SMs wrote
 // visible.  Every wait is bounded: one that runs out raises an abort word that all CTAs
-// see in theirs, sets a flag for the host and ends the kernel.  The first wait of a launch
-// may be long, since other kernels may still hold some of the SMs.
+// see in theirs, sets a flag for the host and ends the kernel.
+//
+// The launch does not need all SMs: another stream's kernel may hold some of them for as long
+// as it likes.  A CTA says that it has started; while some have not kGatherNs after the first
+// stage, those that have go on without them (share_steps below): they deal all nodes out among
+// themselves, with everything read from L2 as a stage launch reads it, and take in the CTAs
+// that start later at every step's end.  A CTA that finds the work done ends at once.  Only a
+// kernel that holds a part of every SM keeps the steps from running until it ends.  With 20 SMs
+// held, us per stage: N=10242 FP64 7.9 (stage launches 4.1; nothing held 3.4 and 4.1), N=40962
+// FP64 12.9 (9.7; 7.2 and 7.7): few warps an SM, for a state that ends with the other kernel.
 //
 // Weights that do not fit (FP64 from N = 27000 to 42600 on 148 SMs) are streamed from L2 in
 // every stage, see kStagePairs.  N=40962: 7.15 us per stage against 8.2 with a launch per
@@ -33,20 +41,38 @@ namespace res {
 
 // threads of a CTA: 16 warps have 128 registers a thread, 20 have 96 (a few of them spilled
 // with FP64)
-constexpr int kFew = 512, kMost = 640;
-constexpr int kSyncWords = 64;         // counter and abort word, a line each
+constexpr int kFewThreads = 512, kMost = 640;
 constexpr int kPt = kPointFields;
-constexpr unsigned long long kWaitNs = 2000000000ull, kFirstWaitNs = 60000000000ull;
+constexpr unsigned long long kWaitNs = 2000000000ull;
+// CTAs of an idle GPU start within a few microseconds of one another, and their first stage
+// comes after about 15 us of loading
+constexpr unsigned long long kGatherNs = 100000ull;
+// a launch runs at most this many steps: the kernels of other streams get a turn every few
+// milliseconds, for less than 1 % in set-up
+constexpr int kLaunchSteps = 200;
+
+// words that the CTAs meet at, zero at launch, each on a line of its own
+enum SyncWord {
+    kArrived = 0,                      // CTAs done with their stages, counted over the launch
+    kAbort = 32,
+    kStarted = 64,                     // CTAs that have started; kShort: they go on without the others
+    kShared = 96,                      // share_steps: CTAs done with their stages of a step
+    kRoster = 128,                     // share_steps, 64 bits: step (from 1) << 32 | CTAs that take part
+    kSyncSet = 160,
+    kSyncWords = 2 * kSyncSet          // the launch's and finish_kernel's
+};
+constexpr unsigned kShort = 1u << 31;
+enum Met { kFailed = 0, kAll = 1, kFew = 2 };
 
 template <typename T>
 struct Args {
     int n, nnbr;
     int m;                             // nodes per CTA
     int nsteps;
-    T *H, *Ka, *Kb;                    // [n][4]
+    T *H, *Ka, *Kb, *D;                // [n][4]; D: share_steps only
     T gh0, c01, c2;                    // c01 = dt/2 (stages 0 and 1), c2 = dt (stage 2)
     double dt6;
-    unsigned* counter;                 // arrivals of the CTAs, zero at launch; abort word 32 words on
+    unsigned* sync;                    // SyncWord
     int* failed;                       // set when a wait ran out (pinned host or device memory)
     unsigned long long wait_ns = kWaitNs;
 };
@@ -125,52 +151,200 @@ __device__ __forceinline__ void get_weights(const float* sw, int m, int slot, in
     w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
 }
 
-// Waits until every CTA has done its `stage`-th stage.
+__device__ __forceinline__ unsigned long long time_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+__device__ __forceinline__ void add_release(unsigned* p) { asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory"); }
+__device__ __forceinline__ unsigned load_acquire(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// One thread: waits until done() holds, looking at the clock and the abort word now and then;
+// aborts when it has waited wait_ns.
+template <typename T, class Done>
+__device__ __forceinline__ bool wait_for(const Args<T>& a, Done done) {
+    unsigned long long t0 = 0;
+    for (unsigned tries = 1; !done(); ++tries) {
+        if (tries & 63) continue;
+        const unsigned long long t = time_ns();
+        if (t0 == 0) t0 = t;
+        if (*(volatile unsigned*)(a.sync + kAbort) != 0 || t - t0 > a.wait_ns) {
+            *(volatile unsigned*)(a.sync + kAbort) = 1;
+            *(volatile int*)a.failed = 1;
+            __threadfence_system();
+            return false;
+        }
+    }
+    return true;
+}
+
+// Waits until every CTA has done its `stage`-th stage: kAll.  After the first stage also kFew,
+// where some CTAs have not started: the bit kShort, which the CTA that gives up waiting sets
+// together with the count of those that have, settles it for all of them -- a CTA that starts
+// later finds it as it says so, and the count can no longer reach the grid's without it.
 template <typename T>
-__device__ __forceinline__ bool exchange(const Args<T>& a, unsigned stage, int* s_ok) {
+__device__ __forceinline__ int exchange(const Args<T>& a, unsigned stage, int* s_met) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.counter) : "memory");
-        volatile unsigned* abort_word = a.counter + 32;
+        add_release(a.sync + kArrived);
         const unsigned all = stage * gridDim.x;
-        unsigned long long t0 = 0;
-        int ok = 1;
-        for (unsigned tries = 1;; ++tries) {
-            unsigned v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.counter) : "memory");
-            if ((int)(v - all) >= 0) break;
-            if ((tries & 63) == 0) {
-                unsigned long long t;
-                asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-                if (t0 == 0) t0 = t;
-                if (*abort_word != 0 || t - t0 > (stage == 1 ? kFirstWaitNs : a.wait_ns)) {
-                    *abort_word = 1;
-                    *(volatile int*)a.failed = 1;
-                    __threadfence_system();
-                    ok = 0;
+        unsigned* started = a.sync + kStarted;
+        auto arrived = [&]() { return (int)(load_acquire(a.sync + kArrived) - all) >= 0; };
+        int met = kAll;
+        if (stage == 1) {
+            const unsigned long long t0 = time_ns();
+            for (unsigned tries = 1; !arrived(); ++tries) {
+                if (tries & 7) continue;
+                const unsigned here = *(volatile unsigned*)started;
+                if (here == gridDim.x) break;                 // none missing: wait for them below
+                if ((here & kShort) ||
+                    (time_ns() - t0 > kGatherNs && atomicCAS(started, here, here | kShort) == here)) {
+                    met = kFew;
                     break;
                 }
             }
         }
-        *s_ok = ok;
+        if (met == kAll && !wait_for(a, arrived)) met = kFailed;
+        *s_met = met;
     }
     __syncthreads();
-    return *s_ok != 0;
+    return *s_met;
+}
+
+// The steps of a launch some of whose CTAs cannot start: CTA `rank` (in the order they started;
+// 0 leads) and the others on the roster take every stage's nodes in turn, a warp's nodes at a
+// time.  Weights, rows and pointwise values are read as a stage launch reads them, base state
+// and accumulator lie in H and D, and the sums have the resident stage's order: the same bits.
+// Those who took part in the first stage have written K rows of this one's first stage, with
+// its values, before they come here.
+template <typename T, int LPN, class Src>
+__device__ __forceinline__ void share_steps(const Args<T>& a, const Src& src, unsigned rank) {
+    constexpr int kNpw = 32 / LPN, kJpl = kSlots / LPN;
+    __shared__ unsigned long long s_roster;
+    __shared__ int s_in, s_go;                               // of the wait for the roster, of a stage's
+    unsigned long long* roster = reinterpret_cast<unsigned long long*>(a.sync + kRoster);
+    unsigned* shared = a.sync + kShared;
+    auto look = [&]() {
+        unsigned long long v;
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(roster) : "memory");
+        return v;
+    };
+    auto publish = [&](unsigned step) {
+        const unsigned long long v = (unsigned long long)step << 32 | (*(volatile unsigned*)(a.sync + kStarted) & ~kShort);
+        asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(roster), "l"(v) : "memory");
+    };
+    const bool wide_h = (reinterpret_cast<uintptr_t>(a.H) & 31) == 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int tl = lane % kNpw, sub = lane / kNpw;
+    if (rank == 0 && threadIdx.x == 0) publish(1);
+    for (unsigned step = 0; step <= (unsigned)a.nsteps;) {
+        // the next step that this CTA is on the roster of, or the end (step nsteps + 1)
+        if (threadIdx.x == 0) {
+            unsigned long long v = 0, before = 0;
+            bool mine = false;
+            do {                                              // the limit starts anew with every step of the others
+                before = v;
+                s_in = wait_for(a, [&]() {
+                    v = look();
+                    mine = (v >> 32) > step && ((unsigned)v > rank || (v >> 32) > (unsigned)a.nsteps);
+                    return mine || v != before;
+                });
+            } while (s_in && !mine);
+            s_roster = v;
+        }
+        __syncthreads();
+        if (!s_in) return;
+        step = (unsigned)(s_roster >> 32);
+        const unsigned few = (unsigned)s_roster;
+        if (step > (unsigned)a.nsteps) return;
+        for (int mode = 0; mode < 4; ++mode) {
+            const T* Kin = mode == kStage0 ? a.H : mode == kStage2 ? a.Kb : a.Ka;
+            T* Kout = mode == kStage3 ? a.H : mode == kStage1 ? a.Kb : a.Ka;
+            const bool wide = mode != kStage0 || wide_h;
+            for (long u = (long)rank * warps + warp; u * kNpw < a.n; u += (long)few * warps) {
+                const long i = u * kNpw + tl, own = min(i, (long)a.n - 1);
+                // the lane's rows at once, then its gathers
+                int rows[kJpl];
+#pragma unroll
+                for (int jj = 0; jj < kJpl; ++jj)
+                    rows[jj] = jj * LPN + sub < a.nnbr ? src.row(own, jj * LPN + sub, a.nnbr, a.n) : (int)own;
+                T acc[16];
+#pragma unroll
+                for (int x = 0; x < 16; ++x) acc[x] = T(0);
+#pragma unroll
+                for (int jj = 0; jj < kJpl; ++jj) {
+                    if (jj * LPN >= a.nnbr) break;
+                    T w[4] = {T(0), T(0), T(0), T(0)}, kv[4];
+                    if (jj * LPN + sub < a.nnbr) src.weights(own, jj * LPN + sub, a.nnbr, w);
+                    load_state(Kin + 4L * rows[jj], wide, kv);
+#pragma unroll
+                    for (int op = 0; op < 4; ++op)
+#pragma unroll
+                        for (int f = 0; f < 4; ++f) acc[op * 4 + f] += w[op] * kv[f];
+                }
+#pragma unroll
+                for (int o = kNpw; o < 32; o <<= 1)
+#pragma unroll
+                    for (int x = 0; x < 16; ++x) acc[x] += __shfl_xor_sync(0xffffffffu, acc[x], o);
+                if (sub != 0 || i >= a.n) continue;
+                T pt[kPointStride], q[4], F[4], h[4], d[4];
+#pragma unroll
+                for (int f = 0; f < kPt; ++f) pt[f] = src.point(i, f);
+                load_state(Kin + 4 * i, wide, q);
+                pointwise_rhs(acc, q, pt, a.gh0, F);
+                if (mode == kStage0) {
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) q[x] = Quad<T>::axpy(q[x], a.c01, F[x]);
+                    lane::put_row(a.D + 4 * i, F);
+                } else {
+                    load_state(a.H + 4 * i, wide_h, h);
+                    load_state(a.D + 4 * i, true, d);
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        d[x] = Quad<T>::axpy(d[x], mode == kStage3 ? T(1) : T(2), F[x]);
+                        q[x] = mode == kStage3 ? Quad<T>::update_h(h[x], a.dt6, d[x])
+                                               : Quad<T>::axpy(h[x], mode == kStage1 ? a.c01 : a.c2, F[x]);
+                    }
+                    if (mode != kStage3) lane::put_row(a.D + 4 * i, d);
+                }
+                if (mode != kStage3 || wide_h) lane::put_row(Kout + 4 * i, q);
+                else Quad<T>::store_row(Kout + 4 * i, q);
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                add_release(shared);
+                s_go = 1;
+                if (mode < 3 || rank == 0)
+                    s_go = wait_for(a, [&]() { return load_acquire(shared) >= few * (unsigned)(mode + 1); });
+                if (mode == 3 && rank == 0 && s_go) {         // all are done: the next step's count and roster
+                    *(volatile unsigned*)shared = 0;
+                    publish(step + 1);
+                }
+            }
+            __syncthreads();
+            if (!s_go) return;
+        }
+    }
 }
 
 // One block that waits, as after a step's second stage, for a block that was never launched:
 // the path of a wait that runs out, without anything to run out of (swe_selftest_step_wait).
 static __global__ void lone_block_kernel(Args<double> a) {
     __shared__ int ok;
-    exchange(a, 2, &ok);
+    exchange(a, 2, &ok);             // (two stages done by a grid of one block)
 }
 
 template <typename T, int LPN, int THREADS, class Src, bool STREAM>
-__global__ void __launch_bounds__(THREADS, 1) steps_kernel(const Args<T> a, const Src src) {
+__global__ void __launch_bounds__(THREADS, 1) steps_kernel(const __grid_constant__ Args<T> a, const __grid_constant__ Src src) {
     constexpr int kNpw = 32 / LPN;          // nodes per warp
     constexpr int kJpl = kSlots / LPN;      // slots per lane
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ int s_ok;
+    __shared__ int s_met;
+    __shared__ unsigned s_started;
     static_assert(!STREAM || (sizeof(T) == 8 && LPN == 2), "streamed weights are FP64, two lanes a node");
     __shared__ __align__(8) uint64_t s_bar[STREAM ? THREADS / 64 : 1];
     const int nst = STREAM ? 2 * kHeldPairs : slots_of(a.nnbr, LPN);   // slots in shared memory
@@ -183,6 +357,7 @@ __global__ void __launch_bounds__(THREADS, 1) steps_kernel(const Args<T> a, cons
     const int tl = lane % kNpw, sub = lane / kNpw;
     const long first = (long)blockIdx.x * a.m;
     const int cnt = (int)min((long)a.m, (long)a.n - first);
+    if (threadIdx.x == 0) s_started = atomicAdd(a.sync + kStarted, 1u);
     // static data of the CTA's nodes
     for (int e = threadIdx.x; e < nst * a.m; e += blockDim.x) {
         const int slot = Src::kNodeFast ? e / a.m : e % nst, ln = Src::kNodeFast ? e % a.m : e / nst;
@@ -232,7 +407,7 @@ __global__ void __launch_bounds__(THREADS, 1) steps_kernel(const Args<T> a, cons
     auto filled = [&]() {
         if constexpr (STREAM) {
             if (!tc::mbar_wait_bounded(bar, batches & 1, kCopyTries)) {
-                *(volatile unsigned*)(a.counter + 32) = 1;
+                *(volatile unsigned*)(a.sync + kAbort) = 1;
                 *(volatile int*)a.failed = 1;
             }
             ++batches;
@@ -353,18 +528,35 @@ __global__ void __launch_bounds__(THREADS, 1) steps_kernel(const Args<T> a, cons
         else Quad<T>::store_row(Kout + 4L * own, q);
     };
 
-    for (int s = 0; s < a.nsteps; ++s) {
+    int met = s_started & kShort ? kFew : kAll;      // the others went on without this CTA
+    for (int s = 0; s < a.nsteps && met == kAll; ++s) {
         const bool last = s + 1 == a.nsteps;
         stage(std::integral_constant<int, kStage0>(), true);
-        if (!exchange(a, ++done, &s_ok)) break;
+        if ((met = exchange(a, ++done, &s_met)) != kAll) break;
         stage(std::integral_constant<int, kStage1>(), true);
-        if (!exchange(a, ++done, &s_ok)) break;
+        if ((met = exchange(a, ++done, &s_met)) != kAll) break;
         stage(std::integral_constant<int, kStage2>(), true);
-        if (!exchange(a, ++done, &s_ok)) break;
+        if ((met = exchange(a, ++done, &s_met)) != kAll) break;
         stage(std::integral_constant<int, kStage3>(), !last);
-        if (!last && !exchange(a, ++done, &s_ok)) break;
+        if (!last) met = exchange(a, ++done, &s_met);
     }
-    if (pending) filled();                 // after an abort: no copy in flight when the block ends
+    if (pending) filled();                 // broken off: no copy in flight when the block ends
+    // (the streamed form has no registers to spare for these: 7.47 us a stage with them at
+    // N=40962, 7.22 without; it leaves the steps to finish_kernel)
+    if constexpr (!STREAM)
+        if (met == kFew) share_steps<T, LPN>(a, src, s_started & ~kShort);
+}
+
+// Follows a launch of the streamed form: nothing to do, unless some of its CTAs could not start.
+constexpr int kFinishThreads = 128, kFinishPerSm = 4;
+template <typename T, int LPN, class Src>
+__global__ void __launch_bounds__(kFinishThreads, kFinishPerSm)
+finish_kernel(const __grid_constant__ Args<T> a, const __grid_constant__ Src src) {
+    __shared__ unsigned s_rank;
+    if (!(a.sync[kStarted - kSyncSet] & kShort)) return;      // a.sync: the second set
+    if (threadIdx.x == 0) s_rank = atomicAdd(a.sync + kStarted, 1u);
+    __syncthreads();
+    share_steps<T, LPN>(a, src, s_rank);
 }
 
 // How a grid of n nodes is split over the SMs with lpn lanes a node: nodes per CTA (a multiple
@@ -388,26 +580,29 @@ inline bool split(int n, int nnbr, int lpn, int sms, size_t smem_max, bool strea
 template <typename T, int LPN, class Src>
 inline cudaError_t launch(const Args<T>& a, const Src& src, int ctas, size_t smem, size_t smem_max, bool stream,
                           cudaStream_t st) {
-    auto kernel = a.m * LPN <= kFew ? steps_kernel<T, LPN, kFew, Src, false> : steps_kernel<T, LPN, kMost, Src, false>;
+    auto kernel = a.m * LPN <= kFewThreads ? steps_kernel<T, LPN, kFewThreads, Src, false> : steps_kernel<T, LPN, kMost, Src, false>;
     if constexpr (Src::kNodeFast && sizeof(T) == 8 && LPN == 2)
         if (stream) kernel = steps_kernel<T, LPN, kMost, Src, true>;
     // the device's limit in every call, never the call's own size: another thread may be
     // between its attribute and its launch
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(a.counter, 0, kSyncWords * sizeof(unsigned), st);
+    e = cudaMemsetAsync(a.sync, 0, kSyncWords * sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas);
     cfg.blockDim = dim3((a.m * LPN + 31) / 32 * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;      // all CTAs resident together, or no launch
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, a, src);
+    e = cudaLaunchKernelEx(&cfg, kernel, a, src);
+    if constexpr (Src::kNodeFast && sizeof(T) == 8 && LPN == 2)
+        if (stream && e == cudaSuccess) {
+            Args<T> rest = a;
+            rest.sync += kSyncSet;
+            finish_kernel<T, LPN, Src><<<ctas * kFinishPerSm, kFinishThreads, 0, st>>>(rest, src);
+            e = cudaGetLastError();
+        }
+    return e;
 }
 
 // shared memory a CTA of the current device may use

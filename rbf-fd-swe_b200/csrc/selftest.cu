@@ -1,4 +1,5 @@
-// Self-test of the bounded waits every pipelined kernel here relies on.
+// Self-tests of the bounded waits every pipelined kernel here relies on, and a kernel that
+// holds SMs for the tests of steps beside one.
 //
 // swe_selftest_wait_timeout launches one block that waits on an mbarrier
 // which nothing ever arrives on, with the time-bounded sleeping wait of the
@@ -30,8 +31,31 @@ __global__ void never_arrives_kernel(unsigned long long limit_ns, int* status, u
     }
 }
 
+__global__ void hold_kernel(unsigned long long limit_ns) {
+    const uint64_t t0 = tc::globaltimer_ns();
+    while (tc::globaltimer_ns() - t0 < limit_ns) __nanosleep(1000);
+}
+
 }  // namespace
 }  // namespace swe
+
+// Blocks that keep an SM each (by its shared memory) for limit_s and wait for nothing else:
+// the long-lived kernel of another stream that a step has to get along with.
+extern "C" int swe_selftest_hold_sms(int blocks, double limit_s, void* stream) {
+    using namespace swe;
+    if (blocks <= 0 || !(limit_s > 0.0) || limit_s > 2.0) {
+        set_error("swe_selftest_hold_sms: need blocks > 0 and a limit in (0, 2] seconds");
+        return SWE_ERR_ARG;
+    }
+    int dev = 0, most = 0;
+    SWE_CUDA_TRY(cudaGetDevice(&dev));
+    SWE_CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    SWE_CUDA_TRY(cudaFuncSetAttribute(hold_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    hold_kernel<<<blocks, 32, most, (cudaStream_t)stream>>>((unsigned long long)(limit_s * 1e9));
+    count_launch();
+    SWE_CUDA_TRY(cudaGetLastError());
+    return SWE_OK;
+}
 
 extern "C" int swe_selftest_wait_timeout(double limit_s, double* waited_s) {
     using namespace swe;

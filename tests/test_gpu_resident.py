@@ -1,6 +1,8 @@
 """Whole steps of the plain form (swe_cuda_step) in the kernel swe_cuda_init chose, resident
 or one launch per stage, on small and mid-sized grids of odd sizes: the bits of the same
 number of swe_cuda_rk_substep rounds, and the oracle's states."""
+import time
+
 import numpy as np
 import pytest
 
@@ -64,8 +66,8 @@ def test_fp32_rhs_of_one_lane_per_node_is_as_exact_as_the_restatement(n):
     ("fp64", 27233, 31, 2, True), ("fp64", 35009, 25, 2, True), ("fp64", 37889, 31, 2, True), ("fp64", 42624, 32, 2, True),
     ("fp32", 1185, 31, 2, False), ("fp32", 20001, 32, 4, False), ("fp32", 47360, 17, 2, False)])
 def test_whole_steps_in_the_resident_kernel_equal_substeps(prec, n, nnbr, lanes, streamed):
-    """The resident kernel, selected: a call is one launch and gives the bits of the stage
-    launches of as many substeps; stage launches when they are selected again."""
+    """The resident kernel, selected: a call is one launch (two where it streams) and gives the
+    bits of the stage launches of as many substeps; stage launches when they are selected again."""
     m = _spiral(n, nnbr)
     m = layout.reorder(m, layout.rcm_mapping(m))
     H0 = m.H_init.astype(np.float64 if prec == "fp64" else np.float32)
@@ -79,7 +81,7 @@ def test_whole_steps_in_the_resident_kernel_equal_substeps(prec, n, nnbr, lanes,
             p.set_state(H0)
             before = capi.kernel_launches()
             p.step(steps)
-            assert capi.kernel_launches() - before == 1
+            assert capi.kernel_launches() - before == (2 if streamed else 1)
             got = p.get_state()
             p.set_state(H0)
             for _ in range(steps):
@@ -155,3 +157,78 @@ def test_init_chooses_the_resident_kernel():
         assert capi.kernel_launches() - before == 1
     finally:
         p.finalize()
+
+
+# blocks of a kernel that holds an SM each, seconds, whether the steps have to end before it does:
+# some SMs held, all but one for a while (the other blocks join as it ends), and all of them
+HELD = [(20, 0.25, True), (147, 0.02, False), (148, 0.02, False)]
+
+
+def _beside(held, seconds, first, run):
+    """run() on its stream while another holds SMs; whether that one still ran at the end."""
+    import torch
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    assert capi.load().swe_selftest_hold_sms(held, seconds, side.cuda_stream) == 0
+    if first:
+        time.sleep(0.02)                            # it has its SMs
+    run()
+    return not side.query()
+
+
+@pytest.mark.parametrize("held,seconds,first", HELD)
+# (every kernel there is: 2 and 4 lanes in blocks of up to 512 and 640 threads, and streamed)
+@pytest.mark.parametrize("prec,n,lanes,steps", [
+    ("fp64", 10242, 4, 40), ("fp64", 23001, 4, 10), ("fp64", 27232, 2, 10), ("fp64", 35009, 2, 10),
+    ("fp32", 10242, 4, 40), ("fp32", 23001, 4, 10), ("fp32", 25001, 2, 20), ("fp32", 40001, 2, 20)])
+def test_steps_run_beside_a_kernel_that_holds_sms(prec, n, lanes, steps, held, seconds, first):
+    """Steps go on, on the SMs that another stream's kernel leaves, while it runs: the bits of the
+    undisturbed steps."""
+    m = _spiral(n, 31)
+    m = layout.reorder(m, layout.rcm_mapping(m))
+    H0 = m.H_init.astype(np.float64 if prec == "fp64" else np.float32)
+    p = capi.Plain()
+    try:
+        p.init_model(m, prec)
+        p.select_step_kernel(lanes)
+        p.set_state(H0)
+        p.step(steps)
+        want = p.get_state()
+        p.set_state(H0)
+        p.sync()
+        got = []
+        running = _beside(held, seconds, first, lambda: (p.step(steps), got.append(p.get_state())))
+        assert running or not first
+        assert np.array_equal(got[0], want)
+    finally:
+        p.finalize()
+
+
+@pytest.mark.parametrize("held,seconds,first", HELD)
+@pytest.mark.parametrize("prec,n,steps,off", [
+    ("fp64", 10242, 40, 2), ("fp64", 20001, 10, 0), ("fp64", 25001, 10, 2), ("fp32", 10242, 20, 0), ("fp32", 20001, 20, 0),
+    ("fp32", 25001, 20, 0), ("fp32", 40001, 20, 0)])
+def test_noalloc_steps_run_beside_a_kernel_that_holds_sms(prec, n, steps, off, held, seconds, first):
+    import torch
+    from test_zz_no_alloc import _call, _device_arrays
+
+    m = _spiral(n, 31)
+    t = _device_arrays(m, prec)
+    buf = torch.empty(4 * n + 2, dtype=torch.float64 if prec == "fp64" else torch.float32, device="cuda")
+    H = buf[off:off + 4 * n].view(n, 4)             # FP64: H 32- and 16-byte aligned
+    H0 = torch.from_numpy(m.H_init).to(H)
+    stream = torch.cuda.Stream()
+
+    def run():
+        _call(m, prec, steps, H, stream.cuda_stream, t)
+        stream.synchronize()
+
+    H.copy_(H0)
+    torch.cuda.synchronize()
+    run()
+    want = H.clone()
+    H.copy_(H0)
+    running = _beside(held, seconds, first, run)
+    assert running or not first
+    assert torch.equal(H, want)
+    _call(m, prec, 0, H, stream.cuda_stream, t)     # no wait ran out
