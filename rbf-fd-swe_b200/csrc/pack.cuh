@@ -87,19 +87,21 @@ __global__ void pack_stencils_kernel(const T* __restrict__ Dx, const T* __restri
 // Cuthill-McKee order): FP64 19.0 / 15.1, FP32 10.9 / 9.4; on a spiral of 30000 nodes FP64
 // 24.7 / 18.5, FP32 17.9 / 12.9.
 //
-// `place` holds up to kPlacedNodes: there two or more lanes share a node, and their sums are
-// as exact as those of the caller's order or more so (FP32 right-hand side of N=40962 against
-// 64 bits: 4.0e-5 in the caller's order, 1.9e-5 placed).  Above, one lane sums a node's 32
-// terms, and the caller's order, nearest first, is the more exact one (N=163842: 1.8e-5
-// against 3.1e-5 placed, 3.6e-5 sorted), at little cost: a stage of N=40962 FP64 takes 8.0 us
+// `place` is for kernels of two or more lanes a node, up to kPlacedNodes: their sums are as
+// exact as in the caller's order or more so (FP32 right-hand side of N=40962 against 64 bits:
+// 4.0e-5 in the caller's order, 1.9e-5 placed).  Where one lane sums a node's 32 terms, the
+// caller's order, nearest first, is the more exact one (N=163842: 1.8e-5 against 3.1e-5 placed,
+// 3.6e-5 sorted), and past kPlacedNodes the gain is small: a stage of N=40962 FP64 takes 8.0 us
 // in the caller's order and 7.2 placed, of 75,000 12.0 and 11.8, of 163,842 28.2 and 28.0,
-// FP32 14.9 and 14.9, of 100,000 11.3 and 10.3.
+// FP32 14.9 and 14.9, of 100,000 11.3 and 10.3.  The plain form packs again when the lanes of
+// its kernel change (Plain::order_slots).
 constexpr int kPlacedNodes = 148 * 5 * (kLaneThreads / 2);   // two lanes a node at 5 CTAs per SM fill the GPU once
+inline bool places_slots(long n, int lanes) { return lanes > 1 && n <= kPlacedNodes; }
 template <typename T>
-__global__ void pack_lanes_kernel(const T* __restrict__ Dx, const T* __restrict__ Dy, const T* __restrict__ Dz,
-                                  const T* __restrict__ L, const int* __restrict__ idx_raw, CallerLayout cl, int n,
-                                  long npad, int nnbr, int rows, int pid0, bool place, T* __restrict__ Wl, int* __restrict__ idxl,
+__global__ void pack_lanes_kernel(const T* __restrict__ W, const int* __restrict__ idxp, int n, long npad, int nnbr,
+                                  int pid0, bool place, T* __restrict__ Wl, int* __restrict__ idxl,
                                   short* __restrict__ idxs, int* __restrict__ wide) {
+    constexpr int U = Quad<T>::kUnits, kPerUnit = 16 / (int)sizeof(T);
     constexpr int kGroup = 32 / (int)sizeof(T);      // nodes whose rows fill a pass
     constexpr int kRowsPerLine = 32 / (int)sizeof(T);
     constexpr int kWarps = 8;
@@ -114,10 +116,7 @@ __global__ void pack_lanes_kernel(const T* __restrict__ Dx, const T* __restrict_
         // (ties in slot order), or as given
         int p = i < n ? (int)i + pid0 : pid0, pos = lane, src = lane;
         if (i < n) {
-            if (lane < nnbr) {
-                const int q = idx_raw[cl.dm(i, lane)];
-                if (q >= 0 && q < rows) p = q;
-            }
+            p = idxp[(i * 8 + lane % 8) * 4 + lane / 8];
             int rank = lane;
             if (place && lane < nnbr) {
                 rank = 0;
@@ -165,18 +164,30 @@ __global__ void pack_lanes_kernel(const T* __restrict__ Dx, const T* __restrict_
             if (u == t) have[u] = i < n ? s_line[warp][lane] : -1;
         const long b = i / kLaneTile, e = (b * kSlots + pos) * kLaneTile + i % kLaneTile;
         T w[4] = {T(0), T(0), T(0), T(0)};
-        if (i < n && lane < nnbr) {
-            const long dm = cl.dm(i, src);
-            w[0] = Dx[dm]; w[1] = Dy[dm]; w[2] = Dz[dm]; w[3] = L[dm];
-        }
+        if (i < n)
+#pragma unroll
+            for (int op = 0; op < 4; ++op)
+                w[op] = W[(((i * kSlotChunks + src / 8) * U + op / kPerUnit) * 8 + src % 8) * kPerUnit + op % kPerUnit];
 #pragma unroll
         for (int op = 0; op < 4; ++op) Wl[4 * e + op] = w[op];
         idxl[e] = p;
         // 16-bit offset from the node's own row (past n: offset 0)
         const int off = i < n ? p - ((int)i + pid0) : 0;
-        if (off < -32768 || off > 32767) atomicOr(wide, 1);
+        if (wide && (off < -32768 || off > 32767)) atomicOr(wide, 1);
         idxs[e] = (short)off;
     }
+}
+
+// The node-per-lane layout of n nodes from their 8-lanes-per-node layout, for a kernel of
+// `lanes` lanes a node; wide: set where an offset does not fit 16 bits (null: not asked).
+template <typename T>
+inline cudaError_t pack_lanes(const T* W, const int* idx, int n, int nnbr, int pid0, int lanes, T* Wl, int* idxl,
+                              short* idxs, int* wide, cudaStream_t st) {
+    const long npad = ((long)n + kLaneTile - 1) / kLaneTile * kLaneTile, groups = npad * (long)sizeof(T) / 32;
+    pack_lanes_kernel<T><<<(unsigned)((groups + 7) / 8), 256, 0, st>>>(W, idx, n, npad, nnbr, pid0, places_slots(n, lanes),
+                                                                      Wl, idxl, idxs, wide);
+    count_launch();
+    return cudaGetLastError();
 }
 
 // One thread per node (and per place of the last tile).
@@ -228,7 +239,7 @@ inline cudaError_t upload(A** dst, const A* src, size_t count, cudaStream_t st, 
 template <typename T>
 int pack_static_device(const CallerLayout& cl, int n, int rows, int pid0, int nnbr, const T* Dx, const T* Dy,
                        const T* Dz, const T* L, const int* idx, const T* x, const T* y, const T* z, const T* f,
-                       const T* ghm, const T* pu, const T* pv, const T* pw, const T* gg, PackedStatic<T>& out) {
+                       const T* ghm, const T* pu, const T* pv, const T* pw, const T* gg, int lanes, PackedStatic<T>& out) {
     const size_t ndm = (size_t)n * cl.pnbr, nv = (size_t)n * 3;
     const long npad = ((long)n + kLaneTile - 1) / kLaneTile * kLaneTile;
     cudaStream_t st = nullptr;
@@ -279,14 +290,14 @@ int pack_static_device(const CallerLayout& cl, int n, int rows, int pid0, int nn
     if ((e = cudaMallocAsync(reinterpret_cast<void**>(&wide), sizeof(int), st))) return fail(e);
     owned.push_back(wide);
     if ((e = cudaMemsetAsync(wide, 0, sizeof(int), st))) return fail(e);
-    const long threads = (long)n * kSlots, groups = npad * (long)sizeof(T) / 32;
+    const long threads = (long)n * kSlots;
     pack_stencils_kernel<T><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(tDx, tDy, tDz, tL, tidx, cl, n, nnbr,
                                                                               rows, pid0, out.W, out.idx, bad);
-    pack_lanes_kernel<T><<<(unsigned)((groups + 7) / 8), 256, 0, st>>>(tDx, tDy, tDz, tL, tidx, cl, n, npad, nnbr, rows,
-                                                                      pid0, n <= kPlacedNodes, out.Wl, out.idxl, out.idxs, wide);
+    if ((e = cudaGetLastError()) || (e = pack_lanes<T>(out.W, out.idx, n, nnbr, pid0, lanes, out.Wl, out.idxl, out.idxs, wide, st)))
+        return fail(e);
     pack_points_kernel<T><<<(unsigned)((npad + 255) / 256), 256, 0, st>>>(tx, ty, tz, tf, tghm, tpu, tpv, tpw, tgg, cl,
                                                                          n, npad, out.PT, out.PTl);
-    count_launch(3);
+    count_launch(2);
     unsigned long long hb = ULLONG_MAX;
     int hw = 1;
     if ((e = cudaGetLastError()) || (e = cudaMemcpyAsync(&hb, bad, sizeof(hb), cudaMemcpyDeviceToHost, st)) ||

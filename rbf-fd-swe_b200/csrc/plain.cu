@@ -110,6 +110,7 @@ struct Plain {
     int kernel_choice = 0;          // 0 = bulk-copy pipelined, 1 = register-streaming, 2 = node-per-lane kernel
     float tune_us[3] = {0.f, 0.f, 0.f};  // stage launch time of each kernel at init (its best shape)
     int lane_lpn = 1;               // node-per-lane kernel: lanes per node (1, 2, 4)
+    bool slots_placed = false;      // its slots are in the order for 2 or 4 lanes (pack_lanes)
     int lane_pf = 0;                // node-per-lane kernel: bulk L2 prefetch at warp start
     int lane_minb = 4;              // node-per-lane kernel: CTAs per SM of its register bound (3, 4, 5)
     int tma_tile = 64;              // pipelined kernel: nodes per tile (64: 1 CTA/SM, 32: 2 CTAs/SM)
@@ -380,7 +381,23 @@ struct Plain {
         return SWE_OK;
     }
 
+    // Packs the node-per-lane layout again where the kernels of `lanes` lanes a node want the
+    // other slot order.  Synchronises on both sides: a stage kernel reads it before its wait for
+    // the launch in front of it.
+    int order_slots(int lanes) {
+        if (places_slots(n, lanes) == slots_placed) return SWE_OK;
+        SWE_CUDA_TRY(cudaStreamSynchronize(stream));
+        if (fsize == 8)
+            SWE_CUDA_TRY(pack_lanes<double>((const double*)W, idx, n, nnbr, pid0, lanes, (double*)Wl, idxl, idxs, nullptr, stream));
+        else
+            SWE_CUDA_TRY(pack_lanes<float>((const float*)W, idx, n, nnbr, pid0, lanes, (float*)Wl, idxl, idxs, nullptr, stream));
+        SWE_CUDA_TRY(cudaStreamSynchronize(stream));
+        slots_placed = places_slots(n, lanes);
+        return SWE_OK;
+    }
+
     int build_graph() {
+        SWE_TRY(order_slots(lane_lpn));
         cudaGraph_t g;
         SWE_CUDA_TRY(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         const bool was = timing;
@@ -436,9 +453,10 @@ static int upload_static(Plain& P, const void* x, const void* y, const void* z, 
                          const void* Dx, const void* Dy, const void* Dz, const void* L) {
     // the caller's arrays go to the device once; every device layout is packed there (pack.cuh)
     PackedStatic<T> ps;
+    P.slots_placed = places_slots(P.n, P.lane_lpn);
     SWE_TRY(pack_static_device<T>(P.cl, P.n, P.rows, P.pid0, P.nnbr, (const T*)Dx, (const T*)Dy, (const T*)Dz,
                                   (const T*)L, idx, (const T*)x, (const T*)y, (const T*)z, (const T*)f,
-                                  (const T*)ghm, (const T*)pu, (const T*)pv, (const T*)pw, (const T*)gg, ps));
+                                  (const T*)ghm, (const T*)pu, (const T*)pv, (const T*)pw, (const T*)gg, P.lane_lpn, ps));
     P.W = ps.W;
     P.idx = ps.idx;
     P.Wl = ps.Wl;
@@ -619,6 +637,7 @@ int swe_cuda_init(int fsize, int layout, int simd_length, int compute_size, int 
             if (c < 3) { P.kernel_choice = 0; P.tma_tile = cand_tile[c]; }
             else if (c == 3) P.kernel_choice = 1;
             else lane_shape(P, c - kLane0);
+            if (c >= kLane0) SWE_TRY(P.order_slots(P.lane_lpn));
             // stages 0, 1, 2 and, for stage 3, 1 again, chained as a step chains them (none of
             // them writes H, and the tile orders alternate as in a step): one sequence to
             // warm up, then three timed
@@ -682,6 +701,7 @@ int swe_cuda_init(int fsize, int layout, int simd_length, int compute_size, int 
                 if (us_c[bs] > 1.1f * us_c[bl]) continue;
                 SWE_TRY(P.setup_resident(1 << l, fits));
                 if (!fits) continue;
+                SWE_TRY(P.order_slots(1 << l));
                 float ms[2] = {0.f, 0.f};
                 for (int r = 0; r < 4; ++r) {              // 2 and 10 steps, the first pair to warm up
                     SWE_CUDA_TRY(cudaEventRecord(e0, P.stream));

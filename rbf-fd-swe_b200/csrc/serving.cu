@@ -835,7 +835,7 @@ int swe_srv_add_grid(int n, int nnbr, double gh0, double dt, const int* idx, con
     cl.pnbr = nnbr;
     PackedStatic<double> ps;
     const int st = pack_static_device<double>(cl, n, n, 0, nnbr, Dx, Dy, Dz, L, idx, x, y, z, f, ghm, p_u, p_v, p_w,
-                                              gradghm, ps);
+                                              gradghm, kSrvLpn, ps);
     if (st != SWE_OK) return -st;
     Grid G;
     G.n = n; G.nnbr = nnbr; G.gh0 = gh0; G.dt = dt;

@@ -232,3 +232,29 @@ def test_noalloc_steps_run_beside_a_kernel_that_holds_sms(prec, n, steps, off, h
     assert running or not first
     assert torch.equal(H, want)
     _call(m, prec, 0, H, stream.cuda_stream, t)     # no wait ran out
+
+
+@pytest.mark.parametrize("n", [20001, 42600, 47360])
+def test_fp32_rhs_of_one_lane_is_as_exact_on_small_grids(n):
+    """The slot order goes with the lanes that sum it, not with the grid's size alone.  One lane
+    per node reads the caller's order, also where 2 and 4 lanes read placed slots: the
+    restatement's sums with one rounding a term instead of two, so an error below the
+    restatement's (as large as it with placed slots).  Each choice keeps its bits after the
+    others."""
+    m = _spiral(n, 31)
+    m = layout.reorder(m, layout.rcm_mapping(m))
+    K = m.H_init.astype(np.float32)
+    want = oracle.Port(m, "fp64").eval_rhs(K.astype(np.float64))
+    restated = np.linalg.norm(oracle.Port(m, "fp32").eval_rhs(K) - want)
+    bar = {1: 0.95 * restated, 2: 1.25 * restated, 4: 1.25 * restated}
+    p = capi.Plain()
+    try:
+        p.init_model(m, "fp32")
+        first = {}
+        for lanes in (1, 2, 4, 1, 4, 2):
+            p.select_kernel(capi.Plain.lane_shape(lanes, 4))
+            F = p.eval_rhs(K).reshape(-1, 4)
+            assert np.linalg.norm(F - want) <= bar[lanes], lanes
+            assert np.array_equal(F, first.setdefault(lanes, F)), lanes
+    finally:
+        p.finalize()
