@@ -682,10 +682,16 @@ int swe_cuda_init(int fsize, int layout, int simd_length, int compute_size, int 
         SWE_TRY(check_waits());
         // Whole steps in the resident kernel where it is faster than four launches of the
         // stage kernel, with the stage kernel's lanes per node (a step and its four substeps
-        // give the same bits): 2 or 4, whichever of those whose stage kernel is within 10 % of
-        // the best gives the faster steps (stage times come in steps of half a microsecond).  us per stage, stage kernel / resident: FP64 N=2562
-        // 3.1 / 2.8, N=10242 4.1 / 3.6, N=20000 6.2 / 4.7, N=40962 8.2 / 7.2; FP32 N=40962 5.1 / 4.2.  Loading
-        // the static data costs about 15 us a call: res_min_steps steps pay for it.
+        // give the same bits): 2 or 4, whichever of those whose stage kernel is as fast as the
+        // best one gives the faster steps.  As fast: to kNoise, the timing's own noise, since
+        // launches of 3 us are as short as the host's time for one.  (Stage kernels run from a
+        // graph, 18 sizes of 1,000 to 47,000 nodes in FP64 and FP32: the lanes chosen so are
+        // within 2 % of the best, so calls of substeps and of few steps lose nothing; a bound of
+        // 1.03 loses the resident kernel at N=10242 FP32, 3.1 us a stage for 2.8.)
+        // us per stage, stage kernel / resident: FP64 N=2562 3.1 / 2.7, N=10242 4.1 / 3.4,
+        // N=20000 5.6 / 4.6, N=40962 7.7 / 7.2; FP32 N=40962 4.6 / 4.2.  Loading the static
+        // data costs about 15 us a call: res_min_steps steps pay for it.
+        constexpr float kNoise = 1.1f;
         if (best == 2 && compute_pid_s == 0 && patch_size == compute_size) {
             int shape = -1, lpn_best = 0;
             float step_best = 3.92f * us_c[bl], setup_best = 0.f;      // faster by 2 % at least
@@ -698,7 +704,7 @@ int swe_cuda_init(int fsize, int layout, int simd_length, int compute_size, int 
                     }
                 if ((bl - kLane0) % 3 == l) bs = bl;
                 bool fits = false;
-                if (us_c[bs] > 1.1f * us_c[bl]) continue;
+                if (us_c[bs] > kNoise * us_c[bl]) continue;
                 SWE_TRY(P.setup_resident(1 << l, fits));
                 if (!fits) continue;
                 SWE_TRY(P.order_slots(1 << l));
@@ -726,6 +732,7 @@ int swe_cuda_init(int fsize, int layout, int simd_length, int compute_size, int 
             // these steps moved H off its initial zero
             SWE_CUDA_TRY(cudaMemsetAsync(P.H, 0, srow, P.stream));
             lane_shape(P, (shape >= 0 ? shape : bl) - kLane0);
+            if (shape >= 0) P.tune_us[2] = us_c[shape];
             P.res_lpn = 0;
             if (shape >= 0) {
                 bool fits = false;
