@@ -92,8 +92,8 @@ struct DevCtl {          // device-resident control words the host sets by async
 
 constexpr int kThreads = kStageThreads;         // 8 warps x 4 nodes
 static_assert(sizeof(ReqDesc) % 16 == 0 && sizeof(ReqDesc) / 16 <= kStageThreads, "descriptor copy");
-// an idle kernel gives the GPU back after 1 ms: a relaunch costs some ten microseconds, and
-// other work of the process waits for the SMs meanwhile
+// an idle kernel gives the GPU back after 1 to 2 ms: other work of the process waits for the SMs
+// meanwhile.  A relaunch costs a launch and the scheduler's next look (it looks every 50 us).
 constexpr unsigned long long kIdleNs = 1000ull * 1000;
 constexpr unsigned long long kDepNs = 10ull * 1000 * 1000 * 1000;    // default dependency wait limit 10 s
 
@@ -225,8 +225,8 @@ __device__ void serve_lanes(const ReqDesc& r, int stage, long base, long end, lo
     serve_epilogue(r, stage, i, sum, Hm + m * moff, Kin + m * moff, Kout + m * moff, Dm + m * moff);
 }
 
-// Exit is collective: the first CTA that has found the queue empty for kIdleNs
-// raises *exiting; from then on no CTA claims work (items already claimed are
+// Exit is collective: a CTA that has found the queue empty, no item claimed and none under
+// way for kIdleNs raises *exiting; from then on no CTA claims work (items already claimed are
 // finished), so every launch runs at full width and the host relaunches, with
 // *exiting cleared, once the kernel has ended and work is queued again.
 // The queue, its tail and the stop word live in device memory (the host
@@ -242,7 +242,7 @@ serve_kernel(Shared* ctl, const DevCtl* dctl, const Item* __restrict__ ring, lon
     __shared__ int s_ok;
     __shared__ ReqDesc s_req;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    unsigned long long idle_since = globaltimer();
+    unsigned long long idle_since = globaltimer(), seen = 0;   // head when the CTA last looked
     while (true) {
         if (threadIdx.x == 0) {
             long long got = -1;
@@ -254,9 +254,15 @@ serve_kernel(Shared* ctl, const DevCtl* dctl, const Item* __restrict__ ring, lon
                     if (atomicCAS(head, h, h + 1) == h) { got = (long long)h; break; }
                     continue;
                 }
-                if (globaltimer() - idle_since > kIdleNs) {           // idle: end this launch everywhere
-                    atomicExch(exiting, 1);
-                    break;
+                if (globaltimer() - idle_since > kIdleNs) {
+                    // (a small request has items for a few CTAs at a time: the others are idle,
+                    // the kernel is not)
+                    if (h == seen && *(volatile unsigned long long*)items_done == h) {
+                        atomicExch(exiting, 1);                       // end this launch everywhere
+                        break;
+                    }
+                    seen = h;
+                    idle_since = globaltimer();
                 }
                 __nanosleep(2000);
             }

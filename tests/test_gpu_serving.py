@@ -182,3 +182,23 @@ def test_n40962_device_order_requests_match_oracle():
     for (mb, st, seed), H0, out in zip(plan, states, outs):
         for b in range(mb):
             assert rel_err(out[b], port.run(H0[b], st)).max() <= 1e-12, (mb, st, b)
+
+
+def test_a_lone_small_request_keeps_its_kernel(models):
+    """A request whose few items leave most of the kernel's blocks without work runs in one
+    launch: idle blocks end it only when the whole kernel has been idle.  (A hiccup of the
+    scheduler thread of a millisecond may cost one more.)"""
+    m = models[4]
+    srv = capi.Server(1 << 30)
+    try:
+        g = srv.add_grid(m)
+        launches = []
+        for steps in (5, 3000):
+            r = srv.submit(g, _states(m, 1, 7), steps)
+            srv.wait([r])
+            srv.fetch(r)
+            launches.append(srv.stats()["kernel_launches"])
+    finally:
+        srv.stop()
+    print("launches before and after a lone request of 12,000 stages:", launches)
+    assert launches[1] - launches[0] <= 5
