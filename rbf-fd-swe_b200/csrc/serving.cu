@@ -54,8 +54,6 @@ struct Item {            // one queue entry (16 bytes)
 };
 
 struct alignas(16) ReqDesc {   // device table entry of an admitted request
-    const uint4* W;      // grid: packed weights
-    const int4* idx;     // grid: packed stencil indices
     const double* PTl;   // grid: tile-transposed pointwise values
     const double* Wl;    // grid: tile-transposed weights (node-per-lane split)
     const int* idxl;     // grid: tile-transposed stencil indices
@@ -365,9 +363,6 @@ struct Grid {
     int n, nnbr;
     int reach = 0;          // work-item chunks a chunk's stencils reach on either side
     double gh0, dt;
-    void* W = nullptr;
-    int* idx = nullptr;
-    void* PT = nullptr;
     void* PTl = nullptr;
     void* Wl = nullptr;     // tile-transposed copies for the node-per-lane split
     int* idxl = nullptr;
@@ -555,8 +550,6 @@ struct Server {
         free_slots.pop_back();
         const size_t one = ((size_t)G.n * 4 * sizeof(double) * r.members + 255) / 256 * 256;
         ReqDesc d{};
-        d.W = reinterpret_cast<const uint4*>(G.W);
-        d.idx = reinterpret_cast<const int4*>(G.idx);
         d.PTl = reinterpret_cast<const double*>(G.PTl);
         d.Wl = reinterpret_cast<const double*>(G.Wl);
         d.idxl = G.idxl;
@@ -854,15 +847,16 @@ int swe_srv_add_grid(int n, int nnbr, double gh0, double dt, const int* idx, con
                 G.reach = std::max(G.reach, dc);
             }
     }
-    G.W = ps.W;
-    G.idx = ps.idx;
-    G.PT = ps.PT;
     G.PTl = ps.PTl;
     G.Wl = ps.Wl;
     G.idxl = ps.idxl;
-    // the 16-bit offsets are not read here: a second index path in the persistent
-    // kernel raises its register demand past the 128 it runs at
-    cudaFree(ps.idxs);
+    // the layouts of the other kernels are not kept (1.3 KB a node), nor are the 16-bit
+    // offsets: a second index path in the persistent kernel raises its register demand past
+    // the 128 it runs at
+    ps.PTl = nullptr;
+    ps.Wl = nullptr;
+    ps.idxl = nullptr;
+    ps.release();
     std::lock_guard<std::mutex> lock(g_srv->mu);
     g_srv->grids.push_back(G);
     return (int)g_srv->grids.size() - 1;
@@ -1030,9 +1024,6 @@ int swe_srv_stop(void) {
     cudaStreamSynchronize(S->kstream);
     cudaStreamSynchronize(S->cstream);
     for (auto& G : S->grids) {
-        cudaFree(G.W);
-        cudaFree(G.idx);
-        cudaFree(G.PT);
         cudaFree(G.PTl);
         cudaFree(G.Wl);
         cudaFree(G.idxl);

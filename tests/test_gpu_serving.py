@@ -202,3 +202,20 @@ def test_a_lone_small_request_keeps_its_kernel(models):
         srv.stop()
     print("launches before and after a lone request of 12,000 stages:", launches)
     assert launches[1] - launches[0] <= 5
+
+
+def test_a_grid_keeps_only_what_the_kernel_reads():
+    """Device memory of a resident grid: tile-transposed weights, indices and pointwise values
+    (1024 + 128 + 136 bytes a node), not the layouts of the other kernels beside them."""
+    import torch
+    m = swe_input.to_model(gen.generate(6, seed=1, device="cuda"))
+    srv = capi.Server(1 << 30)
+    try:
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        srv.add_grid(m)
+        held = before - torch.cuda.mem_get_info()[0]
+    finally:
+        srv.stop()
+    print("bytes a node:", held / m.N)
+    assert held <= 1288 * m.N + (16 << 20)       # allocations come in 2 MiB pieces
