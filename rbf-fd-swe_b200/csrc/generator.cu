@@ -24,7 +24,7 @@
 //   Hyperviscosity Delta^4: [[s_ij^9, P], [P^T, 0]] w = [[9^2 7^2 5^2 3^2 s_j / rho^8], [0]]
 //     with s the tangent-plane distances (s_j = |(xi_j, eta_j)|).
 // Each system (n + 15 unknowns) is solved by Gauss-Jordan elimination with partial
-// pivoting, one warp per node, the augmented matrix in registers.
+// pivoting, one warp per node, the augmented matrix spread over the lanes' registers.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -284,7 +284,7 @@ __device__ __forceinline__ double ipow(double x, int e) {
     return r;
 }
 
-// One warp solves one node's two systems with the augmented matrix in registers.
+// One warp solves one node's two systems, the augmented matrix in its lanes' values.
 //
 // Lane (g, h), g = lane & 15, h = lane >> 4, holds rows g, g + 16, g + 32 of columns
 // 2 i + h: 3 x 25 values, so the two half-warps share every row and the trailing columns
@@ -299,10 +299,13 @@ __device__ __forceinline__ double ipow(double x, int e) {
 // memory and subtracts it from every other row, used ones included (Gauss-Jordan): the
 // lanes that hold them would idle otherwise, and no back substitution follows.
 //
-// Bound by the FP64 pipe and the latency of the steps' chain (maximum, pivot row through
-// shared memory, reciprocal), at 12 warps per SM by registers.  N=163842, k = 31: 29.6 ms
-// with the matrix in shared memory, one lane per row (each step's updates read and write
-// shared memory); 6.9 ms now.
+// Bound by the latency of the steps' chain (maximum, pivot row through shared memory,
+// reciprocal) and the fetch of the unrolled code: issue slots 42 % busy, FP64 pipe 27 %,
+// stalls per issue 1.9 on fixed latencies, 1.0 on instructions, 0.9 on shared memory
+// (N=40962).  12 warps an SM have 168 registers a thread, and part of the 3 x 25 values
+// spills (888 bytes of stores and 1316 of loads a thread in the compiled code, from L1):
+// 6.9 ms at N=163842, k = 31, against 9.3 ms with 8 warps of 254 registers and no spill, and
+// 29.6 ms with the matrix in shared memory, one lane per row.
 constexpr int kNodesPerCta = 2;               // one warp each
 constexpr int kLoc = 25;                      // columns a lane holds
 constexpr int kPolyRow = 32;                  // first polynomial row / column

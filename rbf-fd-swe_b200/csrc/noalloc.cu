@@ -258,16 +258,14 @@ struct RowMajor {
     }
 };
 
-// Whether the resident kernel's call is shorter than a launch per stage: its set-up, the
-// static data's way into shared memory, takes about 15 us.  us per call, stage launches /
-// resident: 20 steps FP64 N=2562 249 / 256, N=5000 361 / 278, N=10242 530 / 321, N=22000
-// 923 / 486, FP32 N=2562 214 / 228, N=10242 328 / 254, N=40962 881 / 395; 2 steps FP64
-// N=2562 46 / 51, N=5000 55 / 53, FP32 N=10242 52 / 51; 1 step FP64 N=5000 38 / 41, N=10242
-// 49 / 44, FP32 N=10242 37 / 40, N=20000 49 / 44.
-inline bool resident_pays(int n, int nsteps, size_t fsize) {
-    const size_t bytes = (size_t)n * fsize;
-    return bytes >= 80000 || (bytes >= 40000 && nsteps >= 2);
-}
+// Whether a grid steps in the resident kernel: its set-up, the static data's way into shared
+// memory, takes about 15 us.  us per call, stage launches / resident: 20 steps FP64 N=2562 249 /
+// 256, N=5000 361 / 278, N=10242 530 / 321, N=22000 923 / 486, FP32 N=2562 214 / 228, N=10242
+// 328 / 254, N=40962 881 / 395; 2 steps FP64 N=2562 46 / 51, N=5000 55 / 53, FP32 N=10242 52 /
+// 51; 1 step FP64 N=5000 38 / 41, N=10242 49 / 44, FP32 N=10242 37 / 40, N=20000 49 / 44.  By
+// size alone: the two sum the slots in different orders, and the same steps give the same bits
+// in one call or in several.
+inline bool resident_pays(int n, size_t fsize) { return (size_t)n * fsize >= 40000; }
 
 // Whole calls in the resident kernel: false where the grid does not fit it.
 template <typename T>
@@ -349,7 +347,7 @@ int run_noalloc(int n, int nnbr, double gh0, double dt, const int* idx, const vo
     const T dtT = (T)dt;
     a.dt6 = (double)dtT / 6.0;
     cudaError_t e = cudaSuccess;
-    if (resident_pays(n, nsteps, sizeof(T)) && run_resident<T>(a, Ka, Kb, dtT, nsteps, A, stream, e)) {
+    if (resident_pays(n, sizeof(T)) && run_resident<T>(a, Ka, Kb, dtT, nsteps, A, stream, e)) {
         SWE_CUDA_TRY(e);
         return SWE_OK;
     }

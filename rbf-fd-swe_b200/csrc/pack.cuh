@@ -89,7 +89,8 @@ __global__ void pack_stencils_kernel(const T* __restrict__ Dx, const T* __restri
 //
 // `place` is for kernels of two or more lanes a node, up to kPlacedNodes: their sums are as
 // exact as in the caller's order or more so (FP32 right-hand side of N=40962 against 64 bits:
-// 4.0e-5 in the caller's order, 1.9e-5 placed).  Where one lane sums a node's 32 terms, the
+// 4.2e-5 in the caller's order, 2.2e-5 placed; two lanes' FP64 sums of N=10242 against longdouble:
+// 5.2e-8 and, alternately from both ends, 3.3e-8).  Where one lane sums a node's 32 terms, the
 // caller's order, nearest first, is the more exact one (N=163842: 1.8e-5 against 3.1e-5 placed,
 // 3.6e-5 sorted), and past kPlacedNodes the gain is small: a stage of N=40962 FP64 takes 8.0 us
 // in the caller's order and 7.2 placed, of 75,000 12.0 and 11.8, of 163,842 28.2 and 28.0,

@@ -233,3 +233,23 @@ def test_noalloc_calls_from_two_threads_do_not_disturb_each_other():
     for th in threads:
         th.join()
     assert not errors, errors[0]
+
+
+@pytest.mark.parametrize("prec,n", [("fp64", 4999), ("fp64", 5000), ("fp64", 9999), ("fp64", 10000), ("fp32", 9999),
+                                    ("fp32", 10000), ("fp32", 19999)])
+def test_noalloc_steps_give_the_same_bits_in_one_call_or_several(prec, n):
+    """Sizes on both sides of the line between stage launches and the resident kernel."""
+    import torch
+
+    m = _spiral(n, 31)
+    t = _device_arrays(m, prec)
+    H0 = torch.from_numpy(m.H_init).to(torch.float64 if prec == "fp64" else torch.float32).cuda()
+    stream = torch.cuda.current_stream().cuda_stream
+    states = []
+    for calls in ((3,), (1, 1, 1), (2, 1)):
+        H = H0.clone()
+        for steps in calls:
+            _call(m, prec, steps, H, stream, t)
+        states.append(H)
+    assert torch.equal(states[0], states[1])
+    assert torch.equal(states[0], states[2])
