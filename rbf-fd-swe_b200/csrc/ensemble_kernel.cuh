@@ -54,15 +54,17 @@
 // Every mbarrier wait is bounded; a timeout sets an error word and a shared
 // abort flag that makes every role leave its loop.
 //
-// What bounds it: the state, accumulator and pointwise rows of a stage are 20 (m32 of 40,962
-// nodes) to 139 us (m64 of 163,842) of DRAM time, the tensor cores need less; the rest is
-// the converters' chain (wait, gather, split, store) and the epilogue's loads.  Measured for
+// What bounds it: with 64 members of N = 163,842 and 3xTF32 a stage moves 1665 MB (707 MB of
+// them the A image), 255 us at the copy bandwidth, and its 1.36e11 MMA operations take 163 us at
+// half the BF16 rate; with 32 members of N = 40,962 and split FP16 it moves 185 MB, 28 us.
+// Neither unit is saturated: the rest is the converters' chain (wait, gather, split, store) and
+// the epilogue's loads, which share the L1 pipe (most stalls wait for a load).  Measured for
 // one stage, 3xTF32 / FP16 / BF16, us:
 //   N = 163,842, 64 members: 334 / 312 / 312, with overlapped launches and odd stages from
 //   the last tile (the rows the stage before wrote last are still in L2) 328 / 306 / 308,
-//   with two adjacent members a thread in 256-bit accesses 317 / 295 / 289;
+//   with two adjacent members a thread in 256-bit accesses 314-322 / 295 / 290;
 //   N = 40,962, 32 members: 72.2 / 70.2 / 69.5, 68.9 / 67 / 66, 67.8 / 64.7 / 63.7, and with
-//   two converter groups 56.5 / 51.0 / 49.8.
+//   two converter groups 56.4 / 50.8 / 49.7.
 // 64 members a CTA keep one group: two would leave a thread 72 registers, and its eight
 // warps already put two on each scheduler.
 #pragma once

@@ -25,10 +25,11 @@
 // held, us per stage: N=10242 FP64 7.9 (stage launches 4.1; nothing held 3.4 and 4.1), N=40962
 // FP64 12.9 (9.7; 7.2 and 7.7): few warps an SM, for a state that ends with the other kernel.
 //
-// Weights that do not fit (FP64 from N = 27000 to 42600 on 148 SMs) are streamed from L2 in
-// every stage, see kStagePairs.  N=40962: 7.15 us per stage against 8.2 with a launch per
-// stage; 8.4 with plain loads of the nodes that do not fit, 7.9 with a copy per slot and
-// warp, 7.5 with two smaller buffers filled four times a stage.
+// Weights that do not fit (31 neighbours, 148 SMs: FP64 from 27,233 to 42,624 nodes) are streamed
+// from L2 in every stage, see kStagePairs.  N=40962: 7.2 us per stage against 7.7 with a launch
+// per stage; before the pointwise values were transposed 7.15 against 8.2, 8.4 with plain loads
+// of the nodes that do not fit, 7.9 with a copy per slot and warp, 7.5 with two smaller buffers
+// filled four times a stage.
 #pragma once
 
 #include <type_traits>
