@@ -119,9 +119,9 @@ int swe_cuda_halo_unpack(int substep_id, const void* recv_buf);
  * memory; no history output open; no kernel forced by swe_cuda_select_kernel), in
  * kernels of up to 200 steps with a block for every SM; the same bits either way.
  * Kernels of other streams that hold some SMs do not keep the steps from running (on
- * the SMs that are left); one that holds a part of every SM does until it ends, and a
- * program whose such kernel waits for the steps selects stage launches
- * (swe_cuda_select_step_kernel).
+ * the SMs that are left); one that holds a part of every SM does until it ends (a block
+ * needs an SM's shared memory as it is), and a program whose such kernel waits for the
+ * steps selects stage launches (swe_cuda_select_step_kernel).
  * Asynchronous; requires compute_pid_s == 0 and patch_size == compute_size
  * (no halo rows: a patch with halo rows steps by swe_cuda_rk_substep with
  * halo exchanges between substeps). */
@@ -246,10 +246,10 @@ int swe_selftest_wait_timeout(double limit_s, double* waited_s);
  * after a step whose wait ran out, until swe_cuda_init is called again.
  * SWE_ERR_STATE where no resident kernel is set up. */
 int swe_selftest_step_wait(double limit_s);
-/* Launches, on `stream` (a cudaStream_t), `blocks` blocks that take an SM's shared memory
- * each and end after limit_s (0 < limit_s <= 2): another stream's long-lived kernel, for
- * tests of steps that run beside one. */
-int swe_selftest_hold_sms(int blocks, double limit_s, void* stream);
+/* Launches, on `stream` (a cudaStream_t), `blocks` blocks of a warp that take `share` (0 to 1)
+ * of an SM's shared memory each and end after limit_s (0 < limit_s <= 2): another stream's
+ * long-lived kernel, for tests of steps that run beside one. */
+int swe_selftest_hold_sms(int blocks, double share, double limit_s, void* stream);
 
 /* ---------------------------------------------------------------------------
  * Batched-ensemble form (members share one grid; tcgen05 tensor cores)
@@ -400,6 +400,13 @@ int swe_cuda_step_noalloc(int fsize, int n, int nnbr, double gh0, double dt, con
                           const void* x, const void* y, const void* z, const void* f, const void* ghm,
                           const void* p_u, const void* p_v, const void* p_w, const void* gradghm,
                           void* H, int nsteps, void* stream);
+/* The same as stage launches on any grid (its results differ in the order of the sums), for
+ * programs whose own long-lived kernel sits on every SM and waits for the steps. */
+int swe_cuda_step_noalloc_stages(int fsize, int n, int nnbr, double gh0, double dt, const int* idx,
+                                 const void* Dx, const void* Dy, const void* Dz, const void* L,
+                                 const void* x, const void* y, const void* z, const void* f, const void* ghm,
+                                 const void* p_u, const void* p_v, const void* p_w, const void* gradghm,
+                                 void* H, int nsteps, void* stream);
 
 /* ---------------------------------------------------------------------------
  * Host utilities (no device work)

@@ -328,7 +328,7 @@ template <typename T>
 int run_noalloc(int n, int nnbr, double gh0, double dt, const int* idx, const void* Dx, const void* Dy,
                 const void* Dz, const void* L, const void* x, const void* y, const void* z, const void* f,
                 const void* ghm, const void* pu, const void* pv, const void* pw, const void* gg, void* H,
-                int nsteps, cudaStream_t stream) {
+                int nsteps, bool stages, cudaStream_t stream) {
     StaticArrays A;
     SWE_TRY(arrays_of_current_device(A));
     T* Ka = reinterpret_cast<T*>(A.scratch);
@@ -347,7 +347,7 @@ int run_noalloc(int n, int nnbr, double gh0, double dt, const int* idx, const vo
     const T dtT = (T)dt;
     a.dt6 = (double)dtT / 6.0;
     cudaError_t e = cudaSuccess;
-    if (resident_pays(n, sizeof(T)) && run_resident<T>(a, Ka, Kb, dtT, nsteps, A, stream, e)) {
+    if (!stages && resident_pays(n, sizeof(T)) && run_resident<T>(a, Ka, Kb, dtT, nsteps, A, stream, e)) {
         SWE_CUDA_TRY(e);
         return SWE_OK;
     }
@@ -365,16 +365,10 @@ int run_noalloc(int n, int nnbr, double gh0, double dt, const int* idx, const vo
     return SWE_OK;
 }
 
-}  // namespace
-}  // namespace swe
-
-using namespace swe;
-
-extern "C" int swe_cuda_step_noalloc(int fsize, int n, int nnbr, double gh0, double dt, const int* idx,
-                                     const void* Dx, const void* Dy, const void* Dz, const void* L,
-                                     const void* x, const void* y, const void* z, const void* f,
-                                     const void* ghm, const void* p_u, const void* p_v, const void* p_w,
-                                     const void* gradghm, void* H, int nsteps, void* stream) {
+int step_noalloc(int fsize, int n, int nnbr, double gh0, double dt, const int* idx, const void* Dx, const void* Dy,
+                 const void* Dz, const void* L, const void* x, const void* y, const void* z, const void* f,
+                 const void* ghm, const void* p_u, const void* p_v, const void* p_w, const void* gradghm, void* H,
+                 int nsteps, bool stages, void* stream) {
     if (fsize != 8 && fsize != 4) { set_error("swe_cuda_step_noalloc: fsize must be 8 or 4, got %d", fsize); return SWE_ERR_ARG; }
     if (nnbr <= 0 || nnbr > kSlots) { set_error("swe_cuda_step_noalloc: nnbr %d not in 1..%d", nnbr, kSlots); return SWE_ERR_ARG; }
     if (nsteps < 0) { set_error("swe_cuda_step_noalloc: nsteps < 0"); return SWE_ERR_ARG; }
@@ -391,7 +385,30 @@ extern "C" int swe_cuda_step_noalloc(int fsize, int n, int nnbr, double gh0, dou
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     if (nsteps == 0) return report_bad_index(s);
     return fsize == 8 ? run_noalloc<double>(n, nnbr, gh0, dt, idx, Dx, Dy, Dz, L, x, y, z, f, ghm, p_u, p_v, p_w,
-                                            gradghm, H, nsteps, s)
+                                            gradghm, H, nsteps, stages, s)
                       : run_noalloc<float>(n, nnbr, gh0, dt, idx, Dx, Dy, Dz, L, x, y, z, f, ghm, p_u, p_v, p_w,
-                                           gradghm, H, nsteps, s);
+                                           gradghm, H, nsteps, stages, s);
+}
+
+}  // namespace
+}  // namespace swe
+
+using namespace swe;
+
+extern "C" int swe_cuda_step_noalloc(int fsize, int n, int nnbr, double gh0, double dt, const int* idx,
+                                     const void* Dx, const void* Dy, const void* Dz, const void* L,
+                                     const void* x, const void* y, const void* z, const void* f,
+                                     const void* ghm, const void* p_u, const void* p_v, const void* p_w,
+                                     const void* gradghm, void* H, int nsteps, void* stream) {
+    return step_noalloc(fsize, n, nnbr, gh0, dt, idx, Dx, Dy, Dz, L, x, y, z, f, ghm, p_u, p_v, p_w, gradghm, H, nsteps,
+                        false, stream);
+}
+
+extern "C" int swe_cuda_step_noalloc_stages(int fsize, int n, int nnbr, double gh0, double dt, const int* idx,
+                                            const void* Dx, const void* Dy, const void* Dz, const void* L,
+                                            const void* x, const void* y, const void* z, const void* f,
+                                            const void* ghm, const void* p_u, const void* p_v, const void* p_w,
+                                            const void* gradghm, void* H, int nsteps, void* stream) {
+    return step_noalloc(fsize, n, nnbr, gh0, dt, idx, Dx, Dy, Dz, L, x, y, z, f, ghm, p_u, p_v, p_w, gradghm, H, nsteps,
+                        true, stream);
 }

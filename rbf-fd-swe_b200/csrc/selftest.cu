@@ -39,19 +39,19 @@ __global__ void hold_kernel(unsigned long long limit_ns) {
 }  // namespace
 }  // namespace swe
 
-// Blocks that keep an SM each (by its shared memory) for limit_s and wait for nothing else:
-// the long-lived kernel of another stream that a step has to get along with.
-extern "C" int swe_selftest_hold_sms(int blocks, double limit_s, void* stream) {
+// Blocks that keep an SM each, or `share` of it (by the shared memory), for limit_s and wait
+// for nothing else: the long-lived kernel of another stream that a step has to get along with.
+extern "C" int swe_selftest_hold_sms(int blocks, double share, double limit_s, void* stream) {
     using namespace swe;
-    if (blocks <= 0 || !(limit_s > 0.0) || limit_s > 2.0) {
-        set_error("swe_selftest_hold_sms: need blocks > 0 and a limit in (0, 2] seconds");
+    if (blocks <= 0 || !(share >= 0.0) || share > 1.0 || !(limit_s > 0.0) || limit_s > 2.0) {
+        set_error("swe_selftest_hold_sms: need blocks > 0, a share in [0, 1] and a limit in (0, 2] seconds");
         return SWE_ERR_ARG;
     }
     int dev = 0, most = 0;
     SWE_CUDA_TRY(cudaGetDevice(&dev));
     SWE_CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     SWE_CUDA_TRY(cudaFuncSetAttribute(hold_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    hold_kernel<<<blocks, 32, most, (cudaStream_t)stream>>>((unsigned long long)(limit_s * 1e9));
+    hold_kernel<<<blocks, 32, (size_t)(share * most), (cudaStream_t)stream>>>((unsigned long long)(limit_s * 1e9));
     count_launch();
     SWE_CUDA_TRY(cudaGetLastError());
     return SWE_OK;

@@ -164,12 +164,13 @@ def test_init_chooses_the_resident_kernel():
 HELD = [(20, 0.25, True), (147, 0.02, False), (148, 0.02, False)]
 
 
-def _beside(held, seconds, first, run):
-    """run() on its stream while another holds SMs; whether that one still ran at the end."""
+def _beside(held, seconds, first, run, share=1.0):
+    """run() on its stream while another's blocks hold `share` of an SM each; whether that one
+    still ran at the end."""
     import torch
     side = torch.cuda.Stream()
     torch.cuda.synchronize()
-    assert capi.load().swe_selftest_hold_sms(held, seconds, side.cuda_stream) == 0
+    assert capi.load().swe_selftest_hold_sms(held, share, seconds, side.cuda_stream) == 0
     if first:
         time.sleep(0.02)                            # it has its SMs
     run()
@@ -258,3 +259,55 @@ def test_fp32_rhs_of_one_lane_is_as_exact_on_small_grids(n):
             assert np.array_equal(F, first.setdefault(lanes, F)), lanes
     finally:
         p.finalize()
+
+
+@pytest.mark.parametrize("form", ["plain", "noalloc"])
+def test_stage_launches_run_beside_a_kernel_on_every_sm(form):
+    """What a program selects whose own kernel sits on every SM and waits for the steps."""
+    import torch
+    from test_zz_no_alloc import _bind, _device_arrays
+
+    m = _spiral(10242, 31)
+    m = layout.reorder(m, layout.rcm_mapping(m))
+    got = []
+    if form == "plain":
+        p = capi.Plain()
+        p.init_model(m, "fp64")
+        p.select_step_kernel(0)
+        p.set_state(m.H_init)
+        p.sync()
+        run = lambda: (p.step(20), got.append(p.get_state().reshape(-1, 4)))  # noqa: E731
+    else:
+        lib = _bind()
+        lib.swe_cuda_step_noalloc_stages.argtypes = lib.swe_cuda_step_noalloc.argtypes
+        t = _device_arrays(m, "fp64")
+        H = torch.from_numpy(m.H_init).cuda()
+        out = torch.empty((m.N, 4), dtype=torch.float64, pin_memory=True)
+        stream = torch.cuda.Stream()
+
+        def step(steps):
+            assert lib.swe_cuda_step_noalloc_stages(
+                8, m.N, m.Nnbr, float(m.gh0), float(m.dt), t["idx"].data_ptr(),
+                *[t[k].data_ptr() for k in ("Dx", "Dy", "Dz", "L", "x", "y", "z", "f", "ghm", "p_u", "p_v", "p_w",
+                                            "gradghm")], H.data_ptr(), steps, stream.cuda_stream) == 0
+
+        def run():
+            before = capi.kernel_launches()
+            step(20)
+            assert capi.kernel_launches() - before == 80
+            with torch.cuda.stream(stream):
+                out.copy_(H, non_blocking=True)
+            stream.synchronize()
+            got.append(out.numpy())
+
+        step(1)                                     # the first call loads the kernels
+        H.copy_(torch.from_numpy(m.H_init))
+
+    try:
+        # (the no-allocation form's stage kernel takes 6 KB of shared memory a block: an SM split
+        # for none has none to give)
+        assert _beside(148, 0.25, True, run, share=0.0 if form == "plain" else 0.08)
+    finally:
+        if form == "plain":
+            p.finalize()
+    assert scaled_err(got[0], oracle.Port(m, "fp64").run(m.H_init, 20)).max() <= 1e-12
