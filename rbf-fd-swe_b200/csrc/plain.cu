@@ -824,9 +824,11 @@ int swe_cuda_step(int nsteps) {
     if (P.use_tma()) P.err_pending = true;
     int s = 0;
     if (P.res_lpn && !P.hist.active() && nsteps >= P.res_min_steps) {
-        for (; s < nsteps; s += res::kLaunchSteps) SWE_CUDA_TRY(P.launch_resident(std::min(res::kLaunchSteps, nsteps - s)));
+        for (int k; s < nsteps; s += k) {
+            k = std::min(res::kLaunchSteps, nsteps - s);
+            SWE_CUDA_TRY(P.launch_resident(k));
+        }
         P.steps_done += nsteps;
-        s = nsteps;
     }
     for (; s < nsteps; ++s) {
         SWE_CUDA_TRY(cudaGraphLaunch(P.graph, P.stream));

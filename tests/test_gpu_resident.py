@@ -123,6 +123,41 @@ def test_resident_rows_of_both_widths(prec, n, lanes):
         p.finalize()
 
 
+@pytest.mark.parametrize("form", ["plain", "noalloc"])
+def test_long_calls_run_in_launches_of_200_steps(form):
+    """A call of 401 steps is three launches and gives the state of calls of 1, 200 and 200."""
+    import torch
+    from test_zz_no_alloc import _call, _device_arrays
+
+    m = _spiral(5921, 31)
+    m = layout.reorder(m, layout.rcm_mapping(m))
+    p = capi.Plain()
+    try:
+        if form == "plain":
+            p.init_model(m, "fp64")
+            p.select_step_kernel(4)
+            start, step, state = lambda: p.set_state(m.H_init), p.step, p.get_state
+        else:
+            t = _device_arrays(m, "fp64")
+            H, stream = torch.from_numpy(m.H_init).cuda(), torch.cuda.current_stream().cuda_stream
+            start = lambda: H.copy_(torch.from_numpy(m.H_init))  # noqa: E731
+            step = lambda n: _call(m, "fp64", n, H, stream, t)  # noqa: E731
+            state = lambda: H.cpu().numpy()  # noqa: E731
+        got = []
+        for calls, launches in (((401,), 3), ((1, 200, 200), 3), ((200, 201), 3)):
+            start()
+            before = capi.kernel_launches()
+            for n in calls:
+                step(n)
+            assert capi.kernel_launches() - before == launches
+            got.append(state())
+        assert np.isfinite(got[0]).all()
+        assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+    finally:
+        if form == "plain":
+            p.finalize()
+
+
 def test_step_kernel_selection_refuses_what_does_not_fit():
     m = _spiral(25001, 31)
     p = capi.Plain()
